@@ -12,9 +12,14 @@
 //    (src/rpoly.h:151-158, 163-173) are capped; hitting the cap sets
 //    kStatusRootLimit and reports the polynomial as having no roots
 //    (ccd_jt.h).
+//
+// The routines that several kernels call per row are out of line and their
+// loops rolled: a kernel's copies of them, inlined and unrolled, exceeded the
+// SM's instruction cache (edge-edge build kernel 185 -> 90 KB).
 #pragma once
 
 #include "ccd_common.h"
+#include "ccd_div.h"
 #include "ccd_math.h"
 #include "ccd_jt.h"
 
@@ -78,7 +83,7 @@ CCD_UNROLL
 
 // ------------------------------------------------------------------ quadratics
 // CTCD::getQuadRoots (src/CTCD.cpp:38-56).
-CCD_HD int quad_roots(double a, double b, double c, double &t0, double &t1) {
+CCD_NOINLINE int quad_roots(double a, double b, double c, double &t0, double &t1) {
   int sign = (b < 0) ? -1 : 1;
   double disc = b * b - 4 * a * c;
   if (disc >= 0) {
@@ -96,13 +101,14 @@ CCD_HD int quad_roots(double a, double b, double c, double &t0, double &t1) {
 }
 
 // CTCD::checkInterval (src/CTCD.cpp:59-79).
-CCD_HD void keep_if_sign(double t1, double t2, const double *op, int degree, SpanList &out, bool want_pos) {
+CCD_NOINLINE void keep_if_sign(double t1, double t2, const double *op, int degree, SpanList &out, bool want_pos) {
   t1 = smax(0.0, t1);
   t2 = smax(0.0, t2);
   t1 = smin(1.0, t1);
   t2 = smin(1.0, t2);
   double tm = (t2 + t1) / 2;
   double f = op[0];
+CCD_ROLLED
   for (int i = 1; i <= degree; i++) {
     f *= tm;
     f += op[i];
@@ -111,9 +117,10 @@ CCD_HD void keep_if_sign(double t1, double t2, const double *op, int degree, Spa
 }
 
 // CTCD::couldHaveRoots (src/CTCD.cpp:81-94).
-CCD_HD bool sign_possible(const double *op, int degree, bool want_pos) {
+CCD_NOINLINE bool sign_possible(const double *op, int degree, bool want_pos) {
   double acc = 0;
   if (want_pos ? (op[0] > 0) : (op[0] < 0)) acc = op[0];
+CCD_ROLLED
   for (int i = 1; i < degree; i++) {
     acc *= 1.0;
     if (want_pos ? (op[i] > 0) : (op[i] < 0)) acc += op[i];
@@ -125,14 +132,17 @@ CCD_HD bool sign_possible(const double *op, int degree, bool want_pos) {
 
 // std::sort on <= 16 doubles in libstdc++ is an insertion sort; the same
 // permutation is reproduced for root lists that contain NaN.
-CCD_HD void sort_roots(double *a, int n) {
+CCD_NOINLINE void sort_roots(double *a, int n) {
+CCD_ROLLED
   for (int i = 1; i < n; i++) {
     double v = a[i];
     if (v < a[0]) {
+CCD_ROLLED
       for (int j = i; j > 0; j--) a[j] = a[j - 1];
       a[0] = v;
     } else {
       int j = i;
+CCD_ROLLED
       while (v < a[j - 1]) {
         a[j] = a[j - 1];
         j--;
@@ -153,12 +163,15 @@ CCD_HD void sort_roots(double *a, int n) {
 //   low_degree_spans / root_spans   the two ways the spans are produced.
 
 // Normalises op (degree n) in place and returns the reduced degree.
-CCD_HD int reduce_poly(double *op, int n) {
+CCD_NOINLINE int reduce_poly(double *op, int n) {
   int deg = n;
   double maxval = 0;
+CCD_ROLLED
   for (int i = 0; i <= n; i++) maxval = smax(maxval, fabs(op[i]));
   if (maxval != 0)
-    for (int i = 0; i <= n; i++) op[i] /= maxval;
+CCD_ROLLED
+    for (int i = 0; i <= n; i++) op[i] = exact_div(op[i], maxval);
+CCD_ROLLED
   for (int i = 0; i < n; i++) {
     if (op[i] == 0)
       deg--;
@@ -166,15 +179,17 @@ CCD_HD int reduce_poly(double *op, int n) {
       break;
   }
   if (deg < n)
+CCD_ROLLED
     for (int i = 0; i <= deg; i++) op[i] = op[i + n - deg];
   return deg;
 }
 
 // Spans from `roots` real root parts tr (unsorted; roots <= 0: none found).
-CCD_HD void root_spans(const double *op, int deg, double *tr, int roots, SpanList &out, bool want_pos) {
+CCD_NOINLINE void root_spans(const double *op, int deg, double *tr, int roots, SpanList &out, bool want_pos) {
   if (roots > 0) {
     sort_roots(tr, roots);
     if (tr[0] >= 0) keep_if_sign(0, tr[0], op, deg, out, want_pos);
+CCD_ROLLED
     for (int i = 0; i < roots - 1; i++)
       if (!((tr[i] < 0 && tr[i + 1] < 0) || (tr[i] > 1.0 && tr[i + 1] > 1.0)))
         keep_if_sign(tr[i], tr[i + 1], op, deg, out, want_pos);
@@ -185,7 +200,7 @@ CCD_HD void root_spans(const double *op, int deg, double *tr, int roots, SpanLis
 }
 
 // Spans of a reduced polynomial of degree <= 2.
-CCD_HD void low_degree_spans(const double *op, int deg, SpanList &out, bool want_pos) {
+CCD_NOINLINE void low_degree_spans(const double *op, int deg, SpanList &out, bool want_pos) {
   double tr[2];
   int roots;
   if (deg == 2) {
@@ -265,24 +280,33 @@ CCD_HD void dist_coeffs(v3d x10, v3d x20, v3d x30, v3d v10, v3d v20, v3d v30, do
   op[6] = D * D - dot(E, E) * minD;
 }
 
+// Point i minus point j of a row x of four points at the start (their
+// velocities, end minus start, when `moving`).
+CCD_HD v3d between(const double *x, int i, int j, bool moving) {
+  const v3d a = ld3(x + 3 * i), b = ld3(x + 3 * j);
+  if (!moving) return a - b;
+  return (ld3(x + 12 + 3 * i) - a) - (ld3(x + 12 + 3 * j) - b);
+}
+
 // The polynomials of one vertex-face row (src/CTCD.cpp:423-472): slots 0-2 are
 // the three edge-side cubics (want >= 0), slot 3 the distance sextic (want <= 0).
-// x: q0s..q3s q0e..q3e.
+// x: q0s..q3s q0e..q3e.  Out of line, and one copy of each polynomial's
+// arithmetic with the points picked by index: inlined for every slot, the
+// polynomials alone overflow an SM's instruction cache.
 struct VFPolys {
   static constexpr int kSlots = 4;
   static CCD_HD int degree(int slot) { return slot < 3 ? 3 : 6; }
   static CCD_HD bool want_pos(int slot) { return slot < 3; }
-  static CCD_HD void coeffs(const double *x, double eta, int slot, double *op) {
-    v3d q0s = ld3(x), q1s = ld3(x + 3), q2s = ld3(x + 6), q3s = ld3(x + 9);
-    v3d v0 = ld3(x + 12) - q0s, v1 = ld3(x + 15) - q1s, v2 = ld3(x + 18) - q2s, v3 = ld3(x + 21) - q3s;
-    if (slot == 0)
-      plane_coeffs(q0s - q1s, cross(q3s - q1s, q2s - q1s), q3s - q1s, v0 - v1, cross(v3 - v1, v2 - v1), v3 - v1, op);
-    else if (slot == 1)
-      plane_coeffs(q0s - q2s, cross(q1s - q2s, q3s - q2s), q1s - q2s, v0 - v2, cross(v1 - v2, v3 - v2), v1 - v2, op);
-    else if (slot == 2)
-      plane_coeffs(q0s - q3s, cross(q2s - q3s, q1s - q3s), q2s - q3s, v0 - v3, cross(v2 - v3, v1 - v3), v2 - v3, op);
+  static CCD_NOINLINE void coeffs(const double *x, double eta, int slot, double *op) {
+    // corner a of the face, then b and c: the side through a and b
+    const int a = slot == 3 ? 1 : slot + 1, b = slot == 0 ? 3 : (slot == 3 ? 2 : slot), c = slot == 0 ? 2 : (slot == 1 ? 3 : (slot == 2 ? 1 : 3));
+    const v3d x10 = between(x, 0, a, false), v10 = between(x, 0, a, true);
+    const v3d xb = between(x, b, a, false), vb = between(x, b, a, true);
+    const v3d xc = between(x, c, a, false), vc = between(x, c, a, true);
+    if (slot < 3)
+      plane_coeffs(x10, cross(xb, xc), xb, v10, cross(vb, vc), vb, op);
     else
-      dist_coeffs(q0s - q1s, q2s - q1s, q3s - q1s, v0 - v1, v2 - v1, v3 - v1, eta * eta, op);
+      dist_coeffs(x10, xb, xc, v10, vb, vc, eta * eta, op);
   }
 };
 
@@ -293,19 +317,20 @@ struct EEPolys {
   static constexpr int kSlots = 5;
   static CCD_HD int degree(int slot) { return slot == 0 ? 6 : 4; }
   static CCD_HD bool want_pos(int slot) { return slot != 0; }
-  static CCD_HD void coeffs(const double *x, double eta, int slot, double *op) {
-    v3d q0s = ld3(x), p0s = ld3(x + 3), q1s = ld3(x + 6), p1s = ld3(x + 9);
-    v3d vp0 = ld3(x + 15) - p0s, vp1 = ld3(x + 21) - p1s, vq0 = ld3(x + 12) - q0s, vq1 = ld3(x + 18) - q1s;
+  static CCD_NOINLINE void coeffs(const double *x, double eta, int slot, double *op) {
+    // points of the three differences x10, x20, x30: q0 = 0, p0 = 1, q1 = 2, p1 = 3
+    const int i1 = slot == 0 || slot > 2 ? 1 : 3, j1 = slot == 0 ? 3 : (slot > 2 ? 0 : 2);
+    const int i2 = slot < 2 ? 1 : (slot == 2 ? 0 : (slot == 3 ? 3 : 2));
+    const int j2 = slot < 2 ? 0 : (slot == 2 ? 1 : (slot == 3 ? 2 : 3));
+    const int i3 = slot == 0 ? 3 : (slot == 1 ? 0 : (slot == 2 ? 1 : (slot == 3 ? 2 : 3)));
+    const int j3 = slot < 3 ? 2 : 0;
+    const v3d x10 = between(x, i1, j1, false), v10 = between(x, i1, j1, true);
+    const v3d x20 = between(x, i2, j2, false), v20 = between(x, i2, j2, true);
+    const v3d x30 = between(x, i3, j3, false), v30 = between(x, i3, j3, true);
     if (slot == 0)
-      dist_coeffs(p0s - p1s, p0s - q0s, p1s - q1s, vp0 - vp1, vp0 - vq0, vp1 - vq1, eta * eta, op);
-    else if (slot == 1)
-      bary_coeffs(p1s - q1s, p0s - q0s, q0s - q1s, vp1 - vq1, vp0 - vq0, vq0 - vq1, op);
-    else if (slot == 2)
-      bary_coeffs(p1s - q1s, q0s - p0s, p0s - q1s, vp1 - vq1, vq0 - vp0, vp0 - vq1, op);
-    else if (slot == 3)
-      bary_coeffs(p0s - q0s, p1s - q1s, q1s - q0s, vp0 - vq0, vp1 - vq1, vq1 - vq0, op);
+      dist_coeffs(x10, x20, x30, v10, v20, v30, eta * eta, op);
     else
-      bary_coeffs(p0s - q0s, q1s - p1s, p1s - q0s, vp0 - vq0, vq1 - vp1, vp1 - vq0, op);
+      bary_coeffs(x10, x20, x30, v10, v20, v30, op);
   }
 };
 

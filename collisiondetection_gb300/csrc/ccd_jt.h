@@ -22,6 +22,7 @@
 #pragma once
 
 #include "ccd_common.h"
+#include "ccd_div.h"
 #include "ccd_math.h"
 
 namespace ccd {
@@ -101,12 +102,16 @@ struct FieldState {
   CCD_HD int &I(int f) const { return i[f * stride + g]; }
 };
 
-// Every division of the solver's phases calls one out-of-line copy of the
-// division sequence: the pool kernel runs every phase's code in the warps of
-// one SM at once, and stalls most on instruction fetch; one shared copy in
-// place of 30-odd inline ones measured 10% off the two-sphere step and 3-4%
-// off the headline batch.  The quotient is the IEEE one, as inline.
-CCD_NOINLINE double jt_div(double a, double b) { return a / b; }
+// Every division of the solver's phases calls one out-of-line copy: the pool
+// kernel runs every phase's code in the warps of one SM at once, and stalls
+// most on instruction fetch.  The copy divides on the FP32 and integer pipes
+// (ccd_div.h; the quotient is the IEEE one).  The same stall is why the loops
+// below are kept rolled (their trip counts are run-time degrees of at most 6;
+// unrolled by the compiler they made the pool kernel 1.1 MB of code, now
+// 0.7 MB).  Both together, start and now: 65,537-row edge-edge batch 5.58 ->
+// 4.00 ms, 24 uneven meshes 622 -> 465 ms, 10M-row batches 217.7 -> 199.5 ms
+// (edge-edge) and 75.3 -> 66.9 ms (vertex-face), one query 731 -> 609 us.
+CCD_NOINLINE double jt_div(double a, double b) { return exact_div(a, b); }
 #define JT_DIV(a, b) jt_div((a), (b))
 
 // ---------------------------------------------------------------- primitives
@@ -117,6 +122,7 @@ CCD_NOINLINE void divide(S s, int nn, int src, int dst, double u, double v, int 
   s.D(dst) = bb;
   double aa = s.D(src + 1) - bb * u;
   s.D(dst + 1) = aa;
+CCD_ROLLED
   for (int i = 2; i <= nn; i++) {
     double cc = s.D(src + i) - aa * u - bb * v;
     s.D(dst + i) = cc;
@@ -204,6 +210,7 @@ CCD_NOINLINE void next_k(S s, int type) {
   if (type == 3) {
     s.D(K) = 0.0;
     s.D(K + 1) = 0.0;
+CCD_ROLLED
     for (int i = 2; i < n; i++) s.D(K + i) = s.D(QK + i - 2);
     return;
   }
@@ -212,6 +219,7 @@ CCD_NOINLINE void next_k(S s, int type) {
   if (fabs(a1) <= fabs(ref) * kEps * 10.0) {
     s.D(K) = 0.0;
     s.D(K + 1) = -a7 * s.D(QP);
+CCD_ROLLED
     for (int i = 2; i < n; i++) s.D(K + i) = a3 * s.D(QK + i - 2) - a7 * s.D(QP + i - 1);
     return;
   }
@@ -221,6 +229,7 @@ CCD_NOINLINE void next_k(S s, int type) {
   s.D(A3) = a3;
   s.D(K) = s.D(QP);
   s.D(K + 1) = s.D(QP + 1) - a7 * s.D(QP);
+CCD_ROLLED
   for (int i = 2; i < n; i++) s.D(K + i) = a3 * s.D(QK + i - 2) - a7 * s.D(QP + i - 1) + s.D(QP + i);
 }
 
@@ -342,6 +351,7 @@ CCD_HD void deflate(S s, int nz, double szr, double lzr) {
   s.Z(jpos) = szr;
   n -= nz;
   s.I(N) = n;
+CCD_ROLLED
   for (int i = 0; i <= n; i++) s.D(P + i) = s.D(QP + i);
   if (nz != 1) s.Z(jpos + 1) = lzr;
   if (n <= 2)
@@ -361,6 +371,7 @@ CCD_HD void end_fixed_iteration(S s) {
   s.I(MODE) = kFixed;
   if (++s.I(J) < s.I(L2)) return;
   const int n = s.I(N);
+CCD_ROLLED
   for (int i = 0; i < n; i++) s.D(K + i) = s.D(TEMP + i);
   if (++s.I(CNT) >= 20) {  // no convergence with 20 shifts
     s.I(ROOTS) = s.I(DEG) - n;
@@ -377,6 +388,7 @@ CCD_NOINLINE void after_tries(S s) {
   const int n = s.I(N);
   s.D(U) = s.D(SVU);
   s.D(V) = s.D(SVV);
+CCD_ROLLED
   for (int i = 0; i < n; i++) s.D(K + i) = s.D(SVK + i);
   const int fl = s.I(FLAGS);
   if ((fl & kVpass) && !(fl & kVtried)) {
@@ -398,6 +410,7 @@ CCD_HD void quad_failed(S s) {  // rpoly.h:334-345
     return;
   }
   const int n = s.I(N);
+CCD_ROLLED
   for (int i = 0; i < n; i++) s.D(K + i) = s.D(SVK + i);
   begin_real(s);
 }
@@ -435,6 +448,7 @@ CCD_HD void start(S s, const double *op, int degree) {
   }
   if (n < 1) return;
   s.I(N) = n;
+CCD_ROLLED
   for (int i = 0; i <= n; i++) s.D(P + i) = op[i];
   if (n <= 2)
     finish_low(s);
@@ -450,6 +464,7 @@ CCD_NOINLINE void step_init(S s) {
   const int n = s.I(N);
   const double lo = kSmalno / kEps;
   double maxc = 0.0, minc = kInfin, x, xm, ff, df, dx;
+CCD_ROLLED
   for (int i = 0; i <= n; i++) {
     x = fabs(s.D(P + i));
     if (x > maxc) maxc = x;
@@ -462,9 +477,11 @@ CCD_NOINLINE void step_init(S s) {
     const int l = (int)(cr_log(sc) / 0x1.62e42fefa39efp-1 + 0.5);  // log(sc) / log(2.0)
     const double factor = ldexp(1.0, l);                            // pow(2.0, l), exact
     if (factor != 1.0)
+CCD_ROLLED
       for (int i = 0; i <= n; i++) s.D(P + i) = factor * s.D(P + i);
   }
   double pt[7];
+CCD_ROLLED
   for (int i = 0; i <= n; i++) pt[i] = fabs(s.D(P + i));
   pt[n] = -pt[n];
   x = cr_exp((cr_log(-pt[n]) - cr_log(pt[0])) / (double)n);
@@ -481,6 +498,7 @@ CCD_NOINLINE void step_init(S s) {
     }
     xm = x * 0.1;
     ff = pt[0];
+CCD_ROLLED
     for (int i = 1; i <= n; i++) ff = ff * xm + pt[i];
     if (ff <= 0.0) break;
     x = xm;
@@ -495,6 +513,7 @@ CCD_NOINLINE void step_init(S s) {
     }
     ff = pt[0];
     df = ff;
+CCD_ROLLED
     for (int i = 1; i < n; i++) {
       ff = ff * x + pt[i];
       df = df * x + ff;
@@ -506,14 +525,17 @@ CCD_NOINLINE void step_init(S s) {
   s.D(BND) = x;
   // Derivative as the first K polynomial, then five unshifted steps.
   const int nm1 = n - 1;
+CCD_ROLLED
   for (int i = 1; i < n; i++) s.D(K + i) = JT_DIV((double)(n - i) * s.D(P + i), (double)n);
   s.D(K) = s.D(P);
   const double aa = s.D(P + n), bb = s.D(P + n - 1);
   bool zerok = (s.D(K + n - 1) == 0);
+CCD_ROLLED
   for (int jj = 0; jj < 5; jj++) {
     const double cc = s.D(K + n - 1);
     if (!zerok) {
       const double t = JT_DIV(-aa, cc);
+CCD_ROLLED
       for (int i = 0; i < nm1; i++) {
         const int j = n - i - 1;
         s.D(K + j) = t * s.D(K + j - 1) + s.D(P + j);
@@ -521,6 +543,7 @@ CCD_NOINLINE void step_init(S s) {
       s.D(K) = s.D(P);
       zerok = (fabs(s.D(K + n - 1)) <= fabs(bb) * kEps * 10.0);
     } else {
+CCD_ROLLED
       for (int i = 0; i < nm1; i++) {
         const int j = n - i - 1;
         s.D(K + j) = s.D(K + j - 1);
@@ -529,6 +552,7 @@ CCD_NOINLINE void step_init(S s) {
       zerok = (s.D(K + n - 1) == 0.0);
     }
   }
+CCD_ROLLED
   for (int i = 0; i < n; i++) s.D(TEMP + i) = s.D(K + i);
   s.I(CNT) = 0;
   s.I(MODE) = kFixed;
@@ -566,6 +590,7 @@ CCD_NOINLINE void step_fixed(S s) {
     if (spass || vpass) {
       s.D(SVU) = s.D(U);
       s.D(SVV) = s.D(V);
+CCD_ROLLED
       for (int i = 0; i < n; i++) s.D(SVK + i) = s.D(K + i);
       s.D(XS) = ss;
       s.I(FLAGS) = (vpass ? kVpass : 0) | (spass ? kSpass : 0);
@@ -598,6 +623,7 @@ CCD_NOINLINE void step_quad(S s) {
   const double zm = sqrt(fabs(v));
   double ee = 2.0 * fabs(s.D(QP));
   const double t = -szr * b;
+CCD_ROLLED
   for (int i = 1; i < n; i++) ee = ee * zm + fabs(s.D(QP + i));
   ee = ee * zm + fabs(a + t);
   ee *= (5.0 * kEps + 4.0 * kEps);
@@ -621,6 +647,7 @@ CCD_NOINLINE void step_quad(S s) {
     s.D(U) = u;
     s.D(V) = v;
     divide(s, n, P, QP, u, v, A, B);
+CCD_ROLLED
     for (int i = 0; i < 5; i++) next_k(s, scalars(s));
     s.I(FLAGS) |= kTried;
     s.I(JQ) = 0;
@@ -646,6 +673,7 @@ CCD_NOINLINE void step_real(S s) {
   const double x = s.D(RX);
   double pv = s.D(P);
   s.D(QP) = pv;
+CCD_ROLLED
   for (int i = 1; i <= n; i++) {
     pv = pv * x + s.D(P + i);
     s.D(QP + i) = pv;
@@ -653,6 +681,7 @@ CCD_NOINLINE void step_real(S s) {
   const double mp = fabs(pv);
   const double ms = fabs(x);
   double ee = (kEps / (kEps + kEps)) * fabs(s.D(QP));
+CCD_ROLLED
   for (int i = 1; i <= n; i++) ee = ee * ms + fabs(s.D(QP + i));
   if (mp <= 20.0 * ((kEps + kEps) * ee - kEps * mp)) {
     deflate(s, 1, x, 0.0);
@@ -672,19 +701,23 @@ CCD_NOINLINE void step_real(S s) {
   s.D(OMP) = mp;
   double kv = s.D(K);
   s.D(QK) = kv;
+CCD_ROLLED
   for (int i = 1; i < n; i++) {
     kv = kv * x + s.D(K + i);
     s.D(QK + i) = kv;
   }
   if (fabs(kv) <= fabs(s.D(K + n - 1)) * 10.0 * kEps) {
     s.D(K) = 0.0;
+CCD_ROLLED
     for (int i = 1; i < n; i++) s.D(K + i) = s.D(QK + i - 1);
   } else {
     t = JT_DIV(-pv, kv);
     s.D(K) = s.D(QP);
+CCD_ROLLED
     for (int i = 1; i < n; i++) s.D(K + i) = t * s.D(QK + i - 1) + s.D(QP + i);
   }
   kv = s.D(K);
+CCD_ROLLED
   for (int i = 1; i < n; i++) kv = kv * x + s.D(K + i);
   t = 0.0;
   if (fabs(kv) > fabs(s.D(K + n - 1) * 10.0 * kEps)) t = JT_DIV(-pv, kv);
@@ -713,6 +746,7 @@ CCD_NOINLINE int jt_solve(const double *op, int degree, double *zr, uint8_t &sta
   const jt::LocalState s{&storage};
   jt::start(s, op, degree);
   while (s.I(jt::MODE) != jt::kDone) jt::step(s);
+CCD_ROLLED
   for (int i = 0; i < degree; i++) zr[i] = s.Z(i);
   status |= (uint8_t)s.I(jt::STATUS);
   return s.I(jt::ROOTS);
