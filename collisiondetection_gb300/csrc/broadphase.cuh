@@ -45,7 +45,8 @@ struct MeshTopology {
 
 // Device buffers of one broad-phase call; grown by the caller.
 struct BroadphaseBuffers {
-  int64_t cap_faces = 0, cap_pairs = 0;
+  int64_t cap_faces = 0, cap_verts = 0, cap_pairs = 0;
+  double *vslab = nullptr;                        // [nv][26]   slabs of the vertices (13-DOP)
   // per face / node
   double *lo64 = nullptr, *hi64 = nullptr;        // [13][nf]
   float *face_lo = nullptr, *face_hi = nullptr;   // [13][nf]   outward-rounded FP32 slabs by face
