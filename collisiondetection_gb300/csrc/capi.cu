@@ -112,6 +112,23 @@ int collect_phase(ccd_context *ctx, PhaseEvents &pe) {
   return CCD_OK;
 }
 
+// The scratch with the context's solver options.  CCD_PATH_REFINE_ALL solves
+// every polynomial (classify false).
+static ccd::StageScratch stage_view(const ccd_context *ctx, const StageBuf &stage, bool classify) {
+  ccd::StageScratch view = stage.view;
+  view.classify = classify;
+  view.wave_steps = view.wd ? ctx->opt_wave_steps : 0;
+  view.wave_min_rows = ctx->opt_wave_min_rows;
+  view.pool_budget = ctx->opt_pool_budget;
+  view.warp_finish = ctx->opt_warp_finish;
+  view.shift_after = ctx->opt_shift_after;
+  view.pool_slots = ctx->opt_pool_slots;
+  view.pool_slots_min = ctx->opt_pool_slots_min;
+  view.pool_all = ctx->opt_pool_all;
+  view.pool_phase_sync = ctx->opt_pool_phase_sync;
+  return view;
+}
+
 // Enqueues the kernels of one batch whose buffers are all on the device.
 int enqueue_batch(ccd_context *ctx, const ccd::PrimBatch &b, int path, int32_t *surv, StageBuf &stage,
                   cudaStream_t s, PhaseEvents *pe) {
@@ -133,19 +150,11 @@ int enqueue_batch(ccd_context *ctx, const ccd::PrimBatch &b, int path, int32_t *
   } else if (all) {
     int rc = ensure_stage(ctx, stage, b.n, s);
     if (rc) return rc;
+    const ccd::StageScratch view = stage_view(ctx, stage, false);
+    CCD_CUDA(ccd::clear_queues(view, s));
     CCD_CUDA(ccd::launch_all_rows(b, surv, s));
     if (pe) CCD_CUDA(cudaEventRecord(pe->ev[1], s));
     int launches = 0;
-    ccd::StageScratch view = stage.view;
-    view.wave_steps = view.wd ? ctx->opt_wave_steps : 0;
-    view.wave_min_rows = ctx->opt_wave_min_rows;
-    view.pool_budget = ctx->opt_pool_budget;
-    view.warp_finish = ctx->opt_warp_finish;
-    view.shift_after = ctx->opt_shift_after;
-    view.pool_slots = ctx->opt_pool_slots;
-    view.pool_slots_min = ctx->opt_pool_slots_min;
-    view.pool_all = ctx->opt_pool_all;
-    view.pool_phase_sync = ctx->opt_pool_phase_sync;
     CCD_CUDA(ccd::launch_stages(b, surv, view, ctx->num_sms, s, &launches));
     if (pe) CCD_CUDA(cudaEventRecord(pe->ev[2], s));
     if (pe) pe->stage_launches = launches;
@@ -158,19 +167,11 @@ int enqueue_batch(ccd_context *ctx, const ccd::PrimBatch &b, int path, int32_t *
   } else {
     int rc = ensure_stage(ctx, stage, b.n, s);
     if (rc) return rc;
+    const ccd::StageScratch view = stage_view(ctx, stage, true);
+    CCD_CUDA(ccd::clear_queues(view, s));
     CCD_CUDA(ccd::launch_prims_cull(b, surv, ctx->num_sms, s));
     if (pe) CCD_CUDA(cudaEventRecord(pe->ev[1], s));
     int launches = 0;
-    ccd::StageScratch view = stage.view;
-    view.wave_steps = view.wd ? ctx->opt_wave_steps : 0;
-    view.wave_min_rows = ctx->opt_wave_min_rows;
-    view.pool_budget = ctx->opt_pool_budget;
-    view.warp_finish = ctx->opt_warp_finish;
-    view.shift_after = ctx->opt_shift_after;
-    view.pool_slots = ctx->opt_pool_slots;
-    view.pool_slots_min = ctx->opt_pool_slots_min;
-    view.pool_all = ctx->opt_pool_all;
-    view.pool_phase_sync = ctx->opt_pool_phase_sync;
     CCD_CUDA(ccd::launch_stages(b, surv, view, ctx->num_sms, s, &launches));
     if (pe) CCD_CUDA(cudaEventRecord(pe->ev[2], s));
     if (pe) pe->stage_launches = launches;

@@ -99,7 +99,8 @@ extern "C" int ccd_prim_batch_device_noalloc(int kind, int64_t n, const double *
   cudaStream_t s = (cudaStream_t)stream;
   ccd::BatchCounters *counters = (ccd::BatchCounters *)(d.scratch + kCountersOff);
   int32_t *surv = (int32_t *)(d.scratch + kSurvOff);
-  const ccd::StageScratch stage = ccd::stage_scratch_view(d.scratch + kStageOff, kTileRows);
+  ccd::StageScratch stage = ccd::stage_scratch_view(d.scratch + kStageOff, kTileRows);
+  stage.classify = true;
   const ccd::PrimBatch b{kind, n, rows, eta, eta_count == n && n != 1, hit, t, nullptr, counters};
   if (cudaMemsetAsync(counters, 0, sizeof(ccd::BatchCounters), s) != cudaSuccess) return CCD_ERR_CUDA;
   // The kernels of the batch entry points' cull + refine path: vertex-vertex
@@ -113,7 +114,8 @@ extern "C" int ccd_prim_batch_device_noalloc(int kind, int64_t n, const double *
     e = ccd::launch_prims_cull(b, surv, d.num_sms, s);
     if (e == cudaSuccess) e = ccd::launch_prims_fp64_list(b, surv, d.num_sms, s);
   } else {
-    e = ccd::launch_prims_cull(b, surv, d.num_sms, s);
+    e = ccd::clear_queues(stage, s);
+    if (e == cudaSuccess) e = ccd::launch_prims_cull(b, surv, d.num_sms, s);
     int launches = 0;
     if (e == cudaSuccess) e = ccd::launch_stages(b, surv, stage, d.num_sms, s, &launches);
   }

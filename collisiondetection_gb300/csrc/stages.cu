@@ -28,8 +28,13 @@ StageScratch stage_scratch_view(void *base, int64_t cap) {
   sc.span_n = (uint8_t *)p;
   p += up(kMaxSlots * c);
   sc.queue = (unsigned *)p;
-  p += up((kMaxSlots + 1) * sizeof(unsigned));
+  p += up(kQueueWords * sizeof(unsigned));
   sc.row_status = (uint32_t *)p;
+  p += up(c * sizeof(uint32_t));
+  sc.row_id = (int32_t *)p;
+  p += up(c * sizeof(int32_t));
+  sc.redo = (int32_t *)p;
+  sc.classify = false;
   sc.jcap = 0;
   sc.wd = nullptr;
   sc.wi = nullptr;

@@ -6,11 +6,13 @@
 // (1/64 of the FP32 rate), so masked lanes are expensive.  The refinement is
 // therefore split into kernels over a tile of survivor rows:
 //
-//   stage_build    thread per row: every polynomial of the row in FP64
-//                  (reference expressions), normalised and degree-reduced;
-//                  lists of degree <= 2 are finished here, the others are
-//                  queued per polynomial slot (one queue per slot, so every
-//                  queue holds polynomials of one nominal degree);
+//   stage_build    every polynomial of the row in FP64 (reference
+//                  expressions); rows that their signs decide drop out and
+//                  lists that cannot matter are not solved (ccd_classify.h);
+//                  the others are normalised and degree-reduced, lists of
+//                  degree <= 2 finished, the rest queued per polynomial slot
+//                  (one queue per slot, so every queue holds polynomials of
+//                  one nominal degree);
 //   root solving   the queued polynomials through the Jenkins-Traub state
 //                  machine (ccd_jt.h), in one of two ways:
 //     wavefront    (large batches) wave_start / wave_step: every solver state
@@ -25,7 +27,8 @@
 //                  are in the same phase, refilling finished slots from the
 //                  queues -- lanes stay busy on equal work without any
 //                  block-wide barrier;
-//   stage_combine  thread per row: the interval-overlap decision.
+//   stage_combine  thread per row: the interval-overlap decision, or the
+//                  polynomials that it still needs queued for a second round.
 //
 // The result equals the reference's: every list the reference computes is
 // computed the same way, and the extra lists computed for rows the reference
@@ -33,6 +36,7 @@
 // soon as any list is empty).
 #pragma once
 
+#include "ccd_classify.h"
 #include "ccd_ctcd64.h"
 #include "ccd_jt_shifts.h"
 #include "ccd_jt_warp.h"
@@ -43,18 +47,19 @@ namespace ccd {
 constexpr int kMaxSlots = 5;
 constexpr int kStageThreads = 128;
 // Wavefront defaults (per-context options override them): lock-step steps
-// before the unfinished jobs move to the pool kernel (about 99% of the queued
-// polynomials finish within 40 solver steps, 99.9% within 120), the steps the
-// pool kernel then gives each before the last ones finish one per warp, and
-// the batch size below which the pool kernel alone solves (the wavefront pays
-// a global-memory round trip per step, which only a large batch hides).
-constexpr int kWaveSteps = 48;
-// 0: the pool kernel finishes every job it resumes.  Handing long solves to
-// the one-per-warp finish only pays when few remain: on near-degenerate
-// polynomials (coplanar edges of flat sheets) about 1% of the solves run
-// through all 20 shifts, 12-15 thousand steps each, and the pool's lane
-// packing beats one busy lane per warp by about 9x there.
-constexpr int kPoolBudget = 0;
+// before the unfinished jobs move to the pool kernel (98% of the queued
+// polynomials finish within 48 solver steps, 99.7% within 128), the steps the
+// pool kernel then gives each before the last ones finish one per warp with a
+// stage's shifts tried at once, and the batch size below which the pool kernel
+// alone solves (the wavefront pays a global-memory round trip per step, which
+// only a large batch hides).  With the classification few solves are left past
+// 128 steps, and among them the ones that fail shift after shift (up to 13,000
+// steps in sequence): 10M edge-edge rows take 67 ms and 10M vertex-face rows
+// 33 ms at 64 / 64, 95 and 46 when the pool finishes every solve.  The second
+// round keeps the pool to the end: on flat sheets thousands of its solves fail
+// all their shifts, and packed lanes are the faster way there.
+constexpr int kWaveSteps = 64;
+constexpr int kPoolBudget = 64;
 constexpr int64_t kWaveMinRows = (int64_t)1 << 18;
 // Job lists: one per (working phase, current degree 3..6).
 constexpr int kWaveBins = 16;
@@ -69,9 +74,13 @@ struct StageScratch {
   double *span_l;       // [slot][k < 7][cap]
   double *span_u;       // [slot][k < 7][cap]
   uint8_t *span_n;      // [slot][cap]
-  unsigned *queue;      // [slot] queued polynomials per slot; [kMaxSlots] next job to start
-  uint32_t *row_status; // [cap]
+  unsigned *queue;      // [slot] queued polynomials per slot; [kMaxSlots] next job to start; the same for the
+                        // second round; then the rows kept by stage_build and those of the second round
+  uint32_t *row_status; // [cap]                status bits, and from bit kUnsolvedShift on the unsolved slots
+  int32_t *row_id;      // [cap]                batch row of each tile row
+  int32_t *redo;        // [cap]                tile rows of the second round
   double *roots;        // [slot][k < 6][cap]   roots found by the solver
+  bool classify;        // drop polynomials whose list is not needed (ccd_classify.h)
   // Wavefront solver (null when not attached: the pool kernel then solves
   // every queued polynomial).  Jobs are numbered slot by slot (queue order).
   int64_t jcap;         // kMaxSlots * cap
@@ -93,17 +102,30 @@ struct StageScratch {
   int pool_phase_sync;  // pool kernel: 0, or k: prefer the phase of the SM clock's current 2^k-cycle window
 };
 
+// Bits of row_status: the slots that stage_build left unsolved, and whether
+// the distance polynomial vanishes exactly at t = 0 beside other terms.
+constexpr int kUnsolvedShift = 8;
+constexpr uint32_t kZeroAtStart = 1u << 16;
+// Queue words: per round the queued polynomials of each slot and the words
+// below, then the kept and redo counts.
+constexpr int kQueueNext = kMaxSlots;       // next job to start
+constexpr int kQueueRound = kMaxSlots + 1;  // words of a round
+constexpr int kQueueRows = 2 * kQueueRound;
+constexpr int kQueueRedo = kQueueRows + 1;
+constexpr int kQueueWords = kQueueRows + 2;
+
 // Bytes of the scratch for a tile of `cap` rows: three [slot][7][cap]
 // double arrays (coefficients, span bounds), one [slot][6][cap] double array
 // (roots), a [slot][cap] int32 array, two [slot][cap] byte arrays, the queue
-// words and a [cap] status array, each rounded up to 256 bytes.
+// words and three [cap] word arrays (status, batch row, second round), each
+// rounded up to 256 bytes.
 constexpr size_t kScratchAlign = 256;
 constexpr size_t scratch_up(size_t x) { return (x + kScratchAlign - 1) / kScratchAlign * kScratchAlign; }
 constexpr size_t stage_scratch_bytes(int64_t cap) {
   return scratch_up(kMaxSlots * 7 * (size_t)cap * sizeof(double)) * 3 +
          scratch_up(kMaxSlots * 6 * (size_t)cap * sizeof(double)) + scratch_up(kMaxSlots * (size_t)cap * sizeof(int32_t)) +
-         scratch_up(kMaxSlots * (size_t)cap) * 2 + scratch_up((kMaxSlots + 1) * sizeof(unsigned)) +
-         scratch_up((size_t)cap * sizeof(uint32_t));
+         scratch_up(kMaxSlots * (size_t)cap) * 2 + scratch_up(kQueueWords * sizeof(unsigned)) +
+         scratch_up((size_t)cap * sizeof(uint32_t)) * 3;
 }
 // Carves the scratch arrays out of one allocation of stage_scratch_bytes(cap)
 // (no wavefront solver attached).
@@ -117,12 +139,45 @@ void attach_wave(StageScratch &sc, void *base);
 // of the staged refinement when no FP32 stage runs (CCD_PATH_REFINE_ALL).
 cudaError_t launch_all_rows(const PrimBatch &b, int32_t *list, cudaStream_t s);
 
+// Clears the job queues.  The caller of launch_stages does so before the kernel
+// that makes the survivor list, which the first stage then follows directly.
+inline cudaError_t clear_queues(const StageScratch &sc, cudaStream_t s) {
+  return cudaMemsetAsync(sc.queue, 0, kQueueWords * sizeof(unsigned), s);
+}
+
 // Enqueues build/roots/combine over every tile of the survivor list.
 // Returns the number of kernels launched through *launches.
 cudaError_t launch_stages(const PrimBatch &b, const int32_t *list, const StageScratch &sc, int num_sms,
                           cudaStream_t s, int *launches);
 
 namespace stages {
+
+// Each kernel of a batch reads what the one before it wrote, and in a batch of
+// a few rows every one is over in 2-3 us, less than its launch takes.  So a
+// kernel is launched while the one before still runs (programmatic dependent
+// launch) and waits here, before it reads or writes anything, until that one
+// has completed; only then does it let its own successor start, so at most one
+// launch waits at a time.  (One vertex-face row without a survivor, batches
+// queued back to back: 38 -> 25 us; 200 rows 343 -> 318 us.)
+__device__ __forceinline__ void follow() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
+template <class... P, class... A>
+void launch_next(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // run() returns the last error
+}
 
 __device__ __forceinline__ void store_spans(const StageScratch &sc, int slot, int64_t r, const SpanList &sl) {
   sc.span_n[slot * sc.cap + r] = (uint8_t)sl.n;
@@ -140,58 +195,187 @@ __device__ __forceinline__ void load_spans(const StageScratch &sc, int slot, int
   }
 }
 
+// Slot `slot` of tile row tr with polynomial op (not yet normalised): finishes
+// a list of degree <= 2, drops a polynomial that cannot have the wanted sign
+// (empty list), and queues the others.  Every lane of the warp calls it;
+// `active` lanes have a polynomial.
 template <class Polys>
-__global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const int32_t *__restrict__ list,
-                                                             int64_t tile_begin, StageScratch sc) {
+__device__ __forceinline__ void queue_slot(const StageScratch &sc, int slot, int64_t tr, bool active, double *op) {
   const unsigned lane = threadIdx.x & 31;
+  bool queue = false;
+  int deg = 0;
+  if (active) {
+    const bool pos = Polys::want_pos(slot);
+    deg = reduce_poly(op, Polys::degree(slot));
+    SpanList sl;
+    sl.clear();
+    if (deg > 2) {
+      queue = sign_possible(op, deg, pos);  // otherwise the list stays empty
+    } else {
+      low_degree_spans(op, deg, sl, pos);
+    }
+    if (!queue) store_spans(sc, slot, tr, sl);
+  }
+  const unsigned mask = __ballot_sync(0xffffffffu, queue);
+  if (!mask) return;
+  unsigned base = 0;
+  const int leader = __ffs(mask) - 1;
+  if ((int)lane == leader) base = atomicAdd(&sc.queue[slot], (unsigned)__popc(mask));
+  base = __shfl_sync(0xffffffffu, base, leader);
+  if (queue) {
+    const int64_t j = base + __popc(mask & ((1u << lane) - 1u));
+    for (int k = 0; k <= deg; k++) sc.coef[(slot * 7 + k) * sc.cap + j] = op[k];
+    sc.job_row[slot * sc.cap + j] = (int32_t)tr;
+    sc.job_deg[slot * sc.cap + j] = (uint8_t)deg;
+  }
+}
+
+// A distance sextic whose last two coefficients are this small beside the
+// largest has roots at (or within rounding of) t = 0: features that start in
+// contact with their common plane, as the edges of a flat sheet do.  Such a
+// solve can run through all 20 shifts (some 13,000 steps, against about 20
+// for others), and the row's other lists usually share no time beyond 0, so
+// it waits for them (stage_combine).  On a flat sheet in rigid motion with
+// jitter, 86% of the solver steps of these sextics are saved.
+// (24 meshes, sheets among them: 465 -> 202 ms with it and the classification.)
+constexpr double kDeferTail = 1e-9;
+
+// The decision of ccd_classify.h for one row by a warp; w: the row's words.
+template <class Polys>
+__device__ __forceinline__ cls::Need classify_row(const float *w) {
+  typedef cls::Row<Polys> R;
+  const int lane = threadIdx.x & 31;
+  cls::Need r{false, R::kAll, 0u};
+  bool mirrored;
+  const unsigned open = R::near_contact(w, lane, mirrored);
+  if (__any_sync(0xffffffffu, mirrored)) return r;
+  const unsigned lanes = __ballot_sync(0xffffffffu, open != 0);
+  // Lanes next to one with open cells may be near; the others' sides are not
+  // looked at.
+  const bool look = ((lanes | (lanes << 1) | (lanes >> 1)) >> lane) & 1u;
+  unsigned out = 0, good = 0;
+  if (look) {
+#pragma unroll 1
+    for (int s = 0; s < R::kSides; s++) {
+      bool g;
+      out |= R::outside(w, s, lane, g);
+      good |= (unsigned)g << s;
+    }
+  }
+  const unsigned live = open & ~out;
+  if (!__any_sync(0xffffffffu, live != 0)) {
+    r.miss = true;
+    return r;
+  }
+  const unsigned before = __shfl_up_sync(0xffffffffu, live, 1), after = __shfl_down_sync(0xffffffffu, live, 1);
+  const bool is_near = live || (lane > 0 && (before & 0xf0u)) || (lane < 31 && (after & 0x0fu));
+  const unsigned near = __ballot_sync(0xffffffffu, is_near);
+  if (cls::runs(near) > cls::kRuns) return r;
+  const unsigned bad = __reduce_or_sync(0xffffffffu, is_near ? ~good & ((1u << R::kSides) - 1u) : 0u);
+  r.solve = (1u << R::kDist) | (R::K == 4 ? bad : bad << 1);
+  r.near = near;
+  return r;
+}
+
+// Rows of the tile (survivors of the FP32 stage): those that ccd_classify.h
+// does not decide get a tile row, and the polynomials to solve are queued.
+// A lane forms its row's polynomials in FP64; the warp then goes through its
+// rows, the lanes sharing the 256 cells of one.  (A lane going alone through
+// the cells of its own row made this kernel 95-180 us long for a single row,
+// against 55 with the warp together.)  A small batch is shared out over
+// `spread` warps.
+template <class Polys>
+__global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const int32_t *list, int64_t tile_begin,
+                                                             StageScratch sc, int spread) {
+  follow();
+  typedef cls::Row<Polys> R;
+  constexpr int K = Polys::kSlots;
+  constexpr int kDist = R::kDist;
+  constexpr int kStride = R::kWords | 1;  // odd: the lanes' rows lie in different banks
+  __shared__ float words[kStageThreads * kStride];
+  const unsigned lane = threadIdx.x & 31;
+  float *mine = words + (threadIdx.x & ~31u) * kStride;
   const int64_t count = (int64_t)b.counters->survivors;
   const int64_t end = count < tile_begin + sc.cap ? count : tile_begin + sc.cap;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t warp_base = tile_begin + (int64_t)blockIdx.x * blockDim.x + (threadIdx.x - lane);
-  for (int64_t w = warp_base; w < end; w += stride) {
+  const int64_t share = (end - tile_begin + spread - 1) / spread;
+  const int per = share < 1 ? 1 : (share < 32 ? (int)share : 32);
+  const int64_t nwarps = (int64_t)gridDim.x * (kStageThreads / 32);
+  for (int64_t w = tile_begin + ((int64_t)blockIdx.x * (kStageThreads / 32) + (threadIdx.x >> 5)) * per; w < end;
+       w += nwarps * per) {
     const int64_t r = w + lane;
-    const bool active = r < end;
-    const int64_t tr = r - tile_begin;
+    bool active = (int)lane < per && r < end;
+    const int rows = end - w < per ? (int)(end - w) : per;
     double x[24];
     double eta = 0.0;
+    int64_t i = 0;
+    bool bounded = false;
+    uint32_t unsolved = 0;
     if (active) {
-      const int64_t i = list[r];
+      i = list[r];
       const double *src = b.rows + i * 24;
 #pragma unroll
       for (int j = 0; j < 24; j++) x[j] = __ldg(src + j);
       eta = b.eta_per_row ? __ldg(b.eta + i) : __ldg(b.eta);
-      sc.row_status[tr] = 0;
-    }
-    for (int slot = 0; slot < Polys::kSlots; slot++) {
-      double op[7];
-      bool queue = false;
-      int deg = 0;
-      if (active) {
-        const bool pos = Polys::want_pos(slot);
+      bounded = sc.classify;
+#pragma unroll 1
+      for (int slot = 0; slot < K; slot++) {
+        if (!sc.classify && slot != kDist) continue;
+        double op[7];
         Polys::coeffs(x, eta, slot, op);
-        deg = reduce_poly(op, Polys::degree(slot));
+        if (slot == kDist) {
+          double m = 0.0;
+#pragma unroll
+          for (int k = 0; k <= 6; k++) m = smax(m, fabs(op[k]));
+          if (fabs(op[5]) + fabs(op[6]) <= kDeferTail * m) {
+            unsolved = 1u << (kUnsolvedShift + kDist);
+            bool other = false;
+#pragma unroll
+            for (int k = 1; k < 6; k++) other = other || op[k] != 0.0;
+            if (op[6] == 0.0 && op[0] != 0.0 && other) unsolved |= kZeroAtStart;
+          }
+        }
+        if (sc.classify) bounded = R::put(mine + lane * kStride, slot, op) && bounded;
+      }
+    }
+    __syncwarp();
+    cls::Need need{false, R::kAll, 0u};
+    const unsigned todo = __ballot_sync(0xffffffffu, bounded);
+#pragma unroll 1
+    for (int k = 0; k < rows; k++) {
+      if (!((todo >> k) & 1u)) continue;
+      const cls::Need n = classify_row<Polys>(mine + k * kStride);
+      if ((int)lane == k) need = n;
+    }
+    __syncwarp();
+    if (need.solve != R::kAll) unsolved = (R::kAll & ~need.solve) << kUnsolvedShift;
+    if (need.miss) {
+      b.hit[i] = 0;
+      if (b.status) b.status[i] = 0;
+      active = false;
+    }
+    // Kept rows take consecutive tile rows.
+    const unsigned kept = __ballot_sync(0xffffffffu, active);
+    if (!kept) continue;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(&sc.queue[kQueueRows], (unsigned)__popc(kept));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const int64_t tr = base + __popc(kept & ((1u << lane) - 1u));
+    if (active) {
+      sc.row_status[tr] = unsolved;
+      sc.row_id[tr] = (int32_t)i;
+    }
+#pragma unroll 1
+    for (int slot = 0; slot < K; slot++) {
+      const bool solve = active && !((unsolved >> (kUnsolvedShift + slot)) & 1u);
+      double op[7];
+      if (solve) {
+        Polys::coeffs(x, eta, slot, op);
+      } else if (active && slot != kDist) {
         SpanList sl;
-        sl.clear();
-        if (deg > 2) {
-          queue = sign_possible(op, deg, pos);  // otherwise the list stays empty
-        } else {
-          low_degree_spans(op, deg, sl, pos);
-        }
-        if (!queue) store_spans(sc, slot, tr, sl);
+        cls::stand_in(need.near, sl);
+        store_spans(sc, slot, tr, sl);
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, queue);
-      if (mask) {
-        unsigned base = 0;
-        const int leader = __ffs(mask) - 1;
-        if ((int)lane == leader) base = atomicAdd(&sc.queue[slot], (unsigned)__popc(mask));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (queue) {
-          const int64_t j = base + __popc(mask & ((1u << lane) - 1u));
-          for (int k = 0; k <= deg; k++) sc.coef[(slot * 7 + k) * sc.cap + j] = op[k];
-          sc.job_row[slot * sc.cap + j] = (int32_t)tr;
-          sc.job_deg[slot * sc.cap + j] = (uint8_t)deg;
-        }
-      }
+      queue_slot<Polys>(sc, slot, tr, solve, op);
     }
   }
 }
@@ -274,6 +458,7 @@ struct PoolJobs {
 // each other's FP64 latency.
 template <class Polys, int POOL>
 __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) {
+  follow();
   constexpr int H = POOL / 32;
   static_assert(POOL % 32 == 0 && H >= 1 && H <= 2, "pool of 32 or 64 slots");
   extern __shared__ double pool_d[];
@@ -539,6 +724,7 @@ __device__ __forceinline__ void load_state(const jt::FieldState &fs, jt::LocalSt
 
 template <class Polys>
 __global__ void __launch_bounds__(kWaveThreads) wave_start(StageScratch sc) {
+  follow();
   __shared__ int qbase[kMaxSlots + 1];
   if (threadIdx.x == 0) queue_bases(sc, Polys::kSlots, qbase);
   __syncthreads();
@@ -575,6 +761,7 @@ __global__ void __launch_bounds__(kWaveThreads) wave_start(StageScratch sc) {
 template <class Polys>
 __global__ void __launch_bounds__(kWaveThreads) wave_step(StageScratch sc, const uint32_t *in, const unsigned *cin,
                                                           uint32_t *out, unsigned *cout, unsigned *czero) {
+  follow();
   __shared__ int qbase[kMaxSlots + 1];
   __shared__ int64_t off[kWaveBins + 1];
   if (threadIdx.x == 0) {
@@ -614,6 +801,7 @@ __global__ void __launch_bounds__(kWaveThreads) wave_step(StageScratch sc, const
 template <class Polys>
 __global__ void __launch_bounds__(kWaveThreads) wave_gather_tail(StageScratch sc, const uint32_t *in,
                                                                  const unsigned *cin, unsigned *tcount) {
+  follow();
   int64_t off[kWaveBins + 1];
   list_offsets(cin, off);
   const int64_t total = off[kWaveBins];
@@ -632,6 +820,7 @@ __global__ void __launch_bounds__(kWaveThreads) wave_gather_tail(StageScratch sc
 // different lanes); otherwise lane 0 runs it alone from a private copy.
 template <class Polys>
 __global__ void __launch_bounds__(32) wave_finish(StageScratch sc, const uint32_t *tail, const unsigned *tcount) {
+  follow();
   __shared__ int qbase[kMaxSlots + 1];
   if (threadIdx.x == 0) queue_bases(sc, Polys::kSlots, qbase);
   __syncwarp();
@@ -657,41 +846,128 @@ __global__ void __launch_bounds__(32) wave_finish(StageScratch sc, const uint32_
   }
 }
 
-template <class Polys>
-__global__ void __launch_bounds__(kStageThreads) stage_combine(PrimBatch b, const int32_t *__restrict__ list,
-                                                               int64_t tile_begin, StageScratch sc) {
+// Whether the side lists of a row (every list but the distance's) share a
+// time; beyond: one after t = 0.
+template <int N>
+__device__ __forceinline__ bool sides_meet(const SpanList *l, bool &beyond) {
+  bool meets = false;
+  beyond = false;
+  for (int i = 0; i < l[0].n; i++)
+    for (int j = 0; j < l[1].n; j++) {
+      const double lo1 = smax(l[0].s[i].l, l[1].s[j].l), hi1 = smin(l[0].s[i].u, l[1].s[j].u);
+      if (lo1 > hi1) continue;
+      for (int k = 0; k < l[2].n; k++) {
+        const double lo2 = smax(lo1, l[2].s[k].l), hi2 = smin(hi1, l[2].s[k].u);
+        if (lo2 > hi2) continue;
+        for (int m = 0; m < (N == 4 ? l[N - 1].n : 1); m++) {
+          const double lo = N == 4 ? smax(lo2, l[N - 1].s[m].l) : lo2, hi = N == 4 ? smin(hi2, l[N - 1].s[m].u) : hi2;
+          if (lo > hi) continue;
+          meets = true;
+          if (hi > 0.0) beyond = true;
+        }
+      }
+    }
+  return meets;
+}
+
+// The decision of each kept row.  First round: a row with unsolved slots is
+// decided if what is solved settles it, and goes to the second round if not:
+//   * unsolved distance sextic: the row misses when its side lists share no
+//     time.  Where they share t = 0 alone, the sextic vanishes there exactly
+//     and the edges are parallel there, the sextic's list holds the span
+//     [0, 0], which counts as parallel and rules out every combination that
+//     touches it: the row misses too;
+//   * unsolved sides of an edge-edge row: their replacement holds as long as
+//     no span is parallel (the parallel rule looks at single combinations of
+//     spans).
+//
+// A row that goes on has its unsolved polynomials queued for the second round
+// right here.
+template <class Polys, bool FIRST>
+__global__ void __launch_bounds__(kStageThreads) stage_combine(PrimBatch b, StageScratch sc) {
+  follow();
+  constexpr int K = Polys::kSlots;
+  constexpr int kDist = cls::Row<Polys>::kDist;
   const unsigned lane = threadIdx.x & 31;
-  const int64_t count = (int64_t)b.counters->survivors;
-  const int64_t end = count < tile_begin + sc.cap ? count : tile_begin + sc.cap;
+  const int64_t end = (int64_t)sc.queue[FIRST ? kQueueRows : kQueueRedo];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t warp_base = tile_begin + (int64_t)blockIdx.x * blockDim.x + (threadIdx.x - lane);
+  const int64_t warp_base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x - lane);
   unsigned hits = 0, flags = 0;
   for (int64_t w = warp_base; w < end; w += stride) {
     const int64_t r = w + lane;
+    int64_t tr = 0, i = 0;
+    uint32_t unsolved = 0;
+    bool again = false;
     if (r < end) {
-      const int64_t tr = r - tile_begin;
-      const int64_t i = list[r];
-      SpanList l[Polys::kSlots];
-      for (int slot = 0; slot < Polys::kSlots; slot++) load_spans(sc, slot, tr, l[slot]);
+      tr = FIRST ? r : sc.redo[r];
+      i = sc.row_id[tr];
+      const uint32_t word = sc.row_status[tr];
+      unsolved = FIRST ? (word >> kUnsolvedShift) & ((1u << K) - 1u) : 0u;
+      SpanList l[K];
+      for (int slot = 0; slot < K; slot++) {
+        if ((unsolved >> kDist & 1u) && slot == kDist)
+          l[slot].clear();
+        else
+          load_spans(sc, slot, tr, l[slot]);
+      }
       double t = 0.0;
-      bool h;
-      if constexpr (Polys::kSlots == 4) {
-        h = vf_combine(l[0], l[1], l[2], l[3], t);
+      bool h = false;
+      if constexpr (K == 4) {
+        if (unsolved >> kDist & 1u) {
+          bool beyond;
+          again = sides_meet<3>(l, beyond);
+        } else {
+          h = vf_combine(l[0], l[1], l[2], l[3], t);
+        }
       } else {
         double x[24];
         const double *src = b.rows + i * 24;
 #pragma unroll
         for (int j = 0; j < 24; j++) x[j] = __ldg(src + j);
         SpanList cop, par;
-        ee_split_parallel(x, l[0], cop, par);
-        h = ee_combine(cop, par, l[1], l[2], l[3], l[4], t);
+        if (unsolved >> kDist & 1u) {
+          bool beyond;
+          again = sides_meet<4>(l + 1, beyond);
+          if (again && !beyond && (word & kZeroAtStart)) {
+            l[0].n = 1;
+            l[0].s[0] = Span{0.0, 0.0};
+            ee_split_parallel(x, l[0], cop, par);
+            again = par.n == 0;
+          }
+        } else {
+          ee_split_parallel(x, l[0], cop, par);
+          again = unsolved && par.n > 0;
+          if (!again) h = ee_combine(cop, par, l[1], l[2], l[3], l[4], t);
+        }
       }
-      const uint8_t st = (uint8_t)sc.row_status[tr];
-      b.hit[i] = h;
-      if (h) b.t[i] = t;
-      if (b.status) b.status[i] = st;
-      hits += h;
-      flags += (st != 0);
+      if (!again) {
+        const uint8_t st = (uint8_t)word;
+        b.hit[i] = h;
+        if (h) b.t[i] = t;
+        if (b.status) b.status[i] = st;
+        hits += h;
+        flags += (st != 0);
+      }
+    }
+    if (FIRST && __any_sync(0xffffffffu, again)) {
+      StageScratch next = sc;
+      next.queue = sc.queue + kQueueRound;
+      double x[24];
+      double eta = 0.0;
+      if (again) {
+        sc.redo[atomicAdd(&sc.queue[kQueueRedo], 1u)] = (int32_t)tr;
+        const double *src = b.rows + i * 24;
+#pragma unroll
+        for (int j = 0; j < 24; j++) x[j] = __ldg(src + j);
+        eta = b.eta_per_row ? __ldg(b.eta + i) : __ldg(b.eta);
+      }
+#pragma unroll 1
+      for (int slot = 0; slot < K; slot++) {
+        const bool solve = again && ((unsolved >> slot) & 1u);
+        double op[7];
+        if (solve) Polys::coeffs(x, eta, slot, op);
+        queue_slot<Polys>(next, slot, tr, solve, op);
+      }
     }
   }
   const unsigned hsum = __reduce_add_sync(0xffffffffu, hits);
@@ -702,9 +978,9 @@ __global__ void __launch_bounds__(kStageThreads) stage_combine(PrimBatch b, cons
   }
 }
 
-inline int stage_grid(int64_t work, int num_sms) {
-  int64_t need = (work + kStageThreads - 1) / kStageThreads;
-  int64_t cap = (int64_t)num_sms * 16;
+inline int stage_grid(int64_t work, int num_sms, int per_block = kStageThreads, int per_sm = 16) {
+  int64_t need = (work + per_block - 1) / per_block;
+  int64_t cap = (int64_t)num_sms * per_sm;
   return (int)(need < 1 ? 1 : (need < cap ? need : cap));
 }
 
@@ -717,47 +993,64 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
   static_assert(kPoolSmem + 1024 <= 48 * 1024, "stage_roots needs an opt-in shared-memory attribute");
   cudaError_t e;
   const int64_t tiles = (b.n + sc.cap - 1) / sc.cap;
-  const int grid = stage_grid(sc.cap, num_sms);
+  // No grid is larger than a tile's rows can fill (a batch of a few rows would
+  // otherwise wait for thousands of empty blocks in every launch).
+  const int64_t rows = b.n < sc.cap ? b.n : sc.cap;
+  const int spread = num_sms * 4;
+  const int64_t build_warps = rows < spread ? rows : ((rows + 31) / 32 > spread ? (rows + 31) / 32 : spread);
+  const int build_grid = stage_grid(build_warps, num_sms, kStageThreads / 32);
+  const int grid = stage_grid(rows, num_sms);
   // Five 64-slot warp pools (about 41 KB each) fit one SM's shared memory,
   // ten 32-slot ones (about 21 KB; 168 registers a lane allow 12 warps).
-  const int pool_grid = num_sms * 5, pool32_grid = num_sms * 10;
+  const int pool_grid = stage_grid(rows * Polys::kSlots, num_sms, 1, 5);
+  const int pool32_grid = stage_grid(rows * Polys::kSlots, num_sms, 1, 10);
   const int wave_grid = num_sms * 8;
+  const PoolJobs queued{nullptr, nullptr, 0, nullptr, nullptr};
   for (int64_t tile = 0; tile < tiles; tile++) {
-    e = cudaMemsetAsync(sc.queue, 0, (kMaxSlots + 1) * sizeof(unsigned), s);
-    if (e != cudaSuccess) return e;
-    stage_build<Polys><<<grid, kStageThreads, 0, s>>>(b, list, tile * sc.cap, sc);
+    if (tile > 0) {
+      e = clear_queues(sc, s);
+      if (e != cudaSuccess) return e;
+    }
+    launch_next(stage_build<Polys>, build_grid, kStageThreads, 0, s, b, list, tile * sc.cap, sc, spread);
     if (sc.wd && sc.wave_steps > 0 && b.n >= sc.wave_min_rows) {
       const int steps = sc.wave_steps;
       const int64_t lstride = (int64_t)kWaveBins * sc.jcap;
       // counts: 3 rotating sets, then the tail and spill lengths
       e = cudaMemsetAsync(sc.wcount, 0, (3 * kWaveBins + 2) * sizeof(unsigned), s);
       if (e != cudaSuccess) return e;
-      wave_start<Polys><<<wave_grid, kWaveThreads, 0, s>>>(sc);
+      launch_next(wave_start<Polys>, wave_grid, kWaveThreads, 0, s, sc);
       for (int it = 0; it < steps; it++) {
-        wave_step<Polys><<<wave_grid, kWaveThreads, 0, s>>>(
-            sc, sc.wlist + (it & 1) * lstride, sc.wcount + kWaveBins * (it % 3), sc.wlist + ((it + 1) & 1) * lstride,
-            sc.wcount + kWaveBins * ((it + 1) % 3), sc.wcount + kWaveBins * ((it + 2) % 3));
+        launch_next(wave_step<Polys>, wave_grid, kWaveThreads, 0, s, sc, sc.wlist + (it & 1) * lstride,
+                    sc.wcount + kWaveBins * (it % 3), sc.wlist + ((it + 1) & 1) * lstride,
+                    sc.wcount + kWaveBins * ((it + 1) % 3), sc.wcount + kWaveBins * ((it + 2) % 3));
       }
       unsigned *tcount = sc.wcount + 3 * kWaveBins, *scount = tcount + 1;
-      wave_gather_tail<Polys><<<num_sms, kWaveThreads, 0, s>>>(sc, sc.wlist + (steps & 1) * lstride,
-                                                               sc.wcount + kWaveBins * (steps % 3), tcount);
+      launch_next(wave_gather_tail<Polys>, num_sms, kWaveThreads, 0, s, sc, sc.wlist + (steps & 1) * lstride,
+                  sc.wcount + kWaveBins * (steps % 3), tcount);
       // The unfinished jobs continue in the pool kernel (many per warp); the
       // few that exceed its step budget finish one per warp, as many warps as
       // can be resident at once.  The wavefront lists are free again and hold
       // the spilled jobs.
-      stage_roots<Polys, kWarpPool><<<pool_grid, 32, kPoolSmem, s>>>(
-          sc, PoolJobs{sc.tail, tcount, sc.pool_budget, sc.wlist, scount});
-      wave_finish<Polys><<<num_sms * 32, 32, 0, s>>>(sc, sc.wlist, scount);
+      launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc,
+                  PoolJobs{sc.tail, tcount, sc.pool_budget, sc.wlist, scount});
+      StageScratch last = sc;
+      last.shift_after = sc.shift_after < 1 ? sc.shift_after : 1;
+      launch_next(wave_finish<Polys>, num_sms * 32, 32, 0, s, last, sc.wlist, scount);
       *launches += steps + 4;
     } else {
       if (sc.pool_slots == 32)
-        stage_roots<Polys, 32><<<pool32_grid, 32, pool_smem(32), s>>>(sc, PoolJobs{nullptr, nullptr, 0, nullptr, nullptr});
+        launch_next(stage_roots<Polys, 32>, pool32_grid, 32, pool_smem(32), s, sc, queued);
       else
-        stage_roots<Polys, kWarpPool><<<pool_grid, 32, kPoolSmem, s>>>(sc, PoolJobs{nullptr, nullptr, 0, nullptr, nullptr});
+        launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc, queued);
       *launches += 1;
     }
-    stage_combine<Polys><<<grid, kStageThreads, 0, s>>>(b, list, tile * sc.cap, sc);
-    *launches += 2;
+    launch_next(stage_combine<Polys, true>, grid, kStageThreads, 0, s, b, sc);
+    // Second round: usually few rows or none, so the pool kernel alone.
+    StageScratch sc2 = sc;
+    sc2.queue = sc.queue + kQueueRound;
+    launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc2, queued);
+    launch_next(stage_combine<Polys, false>, grid, kStageThreads, 0, s, b, sc);
+    *launches += 4;
   }
   return cudaGetLastError();
 }

@@ -96,7 +96,7 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *   "wave_steps"     root-solver steps taken in lock-step over all queued
  *                    polynomials of a large batch before the unfinished ones
  *                    continue in the per-warp pool solver (0: the pool
- *                    solver only); default 48, at most 4096
+ *                    solver only); default 64, at most 4096
  *   "wave_min_rows"  smallest batch (rows) that uses those lock-step steps;
  *                    default 262144
  *   "count_slab_tests" 1: the broad phase counts its traversal's slab tests
@@ -118,14 +118,14 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *                    smaller register budget; default 3
  *   "pool_budget"    further steps the unfinished polynomials get, many per
  *                    warp, before the last ones are finished one per warp
- *                    (0: no limit); default 0
+ *                    (0: no limit); default 64
  *   "pool_slots"     pool solver of a batch the wavefront does not take:
  *                    solver slots per warp, 64 (five warps per SM) or 32
  *                    (ten warps per SM); default 64
  *   "pool_slots_min" pool solver: a warp fills its share of the queued
  *                    polynomials (the queue over the grid's warps), but at
  *                    least this many of its 64 slots; a small share spreads
- *                    a small batch over more warps; in [1, 64], default 4
+ *                    a small batch over more warps; in [1, 64], default 1
  *                    (64: the first warps fill all their slots)
  *   "pool_all"       pool solver: once the queue is drained, a warp with at
  *                    most this many solves left advances all of them at
@@ -143,10 +143,10 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *                    1 on all 32 lanes with independent operations spread
  *                    over them, 2 each lane trying one of the stage's
  *                    remaining shifts, the first that converges kept (the
- *                    same results as the sequential order); default 1
+ *                    same results as the sequential order); default 2
  *   "shift_after"    warp_finish 2: shifts of a stage tried one at a time
- *                    before the remaining ones run at once; in [0, 19],
- *                    default 2
+ *                    before the remaining ones run at once (at most 1 by the
+ *                    one-per-warp finish); in [0, 19], default 2
  *   "chunk_rows"     ccd_prim_batch: largest chunk (rows) streamed through
  *                    the device, two in flight; a batch is cut into equal
  *                    chunks; in [1024, 2^26], default 2^23
