@@ -54,6 +54,11 @@ constexpr float kCell = 1.0f / (kLanes * kPer);
 constexpr float kMargin = 1e-5f;
 constexpr float kMirror = 1e-4f;
 constexpr float kRound = 1.5e-6f;    // coefficients and Horner steps in FP32, sum|c| = 1
+// Coefficients further apart than this are left to the solver: with roots 30
+// orders of magnitude apart it can lose one and report a span without the
+// wanted sign (1 in 10^6 rows with coordinates between 1e-20 and 1e20; none in
+// 7 million with this bound).
+constexpr float kLeast = 1e-30f;
 constexpr int kRuns = 3;             // runs of non-empty cells kept; more are left to the solver
 
 // FP32 coefficients (ascending powers, sum|c| = 1) of the degree-N polynomial
@@ -72,9 +77,11 @@ CCD_UNROLL
   double scale;
   memcpy(&scale, &bits, sizeof scale);
   float a[N + 1], s = 0.0f;
+  bool even = true;
 CCD_UNROLL
   for (int i = 0; i <= N; i++) {
     a[i] = (float)(op[N - i] * scale);
+    even = even && (op[N - i] == 0.0 || fabsf(a[i]) > kLeast);
     s += fabsf(a[i]);
   }
   const float r = 1.0f / s;
@@ -101,7 +108,7 @@ CCD_UNROLL
   const float bend = kCell * kCell * 0.13f;  // > h^2 / 8
   p[N + 1] = bend * most + kRound;
   p[N + 2] = bend * sum + kRound;
-  return s == s;
+  return even && s == s;
 }
 
 template <int N>

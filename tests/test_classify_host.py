@@ -106,3 +106,18 @@ def test_takes_no_row_that_it_cannot_bound(kind):
     out, differs, _, _ = _classify(kind, rows[np.r_[0:4000:4, 3:4000:4]], 1e-6)
     assert set(np.unique(out)) <= {0, 4}
     assert differs.sum() == 0
+
+
+def test_leaves_rows_of_far_apart_coefficients_to_the_solver():
+    # coordinates 70 orders of magnitude apart: the solver loses a root of the
+    # second side and reports it positive up to t = 1, which decides the row
+    row = [
+        1.3412941393225036e-09, 7.680402678565238e-30, 1.1797703088715006e-29, 1.6909395566468181e-40,
+        28123401653.643394, 6.661879818881568e-09, 1.2909404345665422e+24, 1.758315190363229e+32,
+        6.990541081300586e-27, 1.0676368764076317e+18, 6.840042438680488e-28, 1.6032392515276564e-06,
+        532036290.6228999, 1.9107187881559787e-34, 7526.8785214051695, 1.132284335397677e-37, 0.42749773874772373,
+        1.6464199379580506e-06, 1.1066387145431088e+26, 0.001784983565492135, 4.324384243362487e+23,
+        1.9697658226502924e-29, 3.344853031520508e-11, 0.001334615982166079,
+    ]
+    out, differs, _, _ = _classify(0, np.array([row]), 1e-6)
+    assert out[0] == 4 and not differs[0]
