@@ -55,12 +55,25 @@ constexpr int kStageThreads = 128;
 // only a large batch hides).  With the classification few solves are left past
 // 128 steps, and among them the ones that fail shift after shift (up to 13,000
 // steps in sequence): 10M edge-edge rows take 67 ms and 10M vertex-face rows
-// 33 ms at 64 / 64, 95 and 46 when the pool finishes every solve.  The second
+// 33 ms at 64 / 64, 95 and 46 when a full pool finishes every solve.  The second
 // round keeps the pool to the end: on flat sheets thousands of its solves fail
 // all their shifts, and packed lanes are the faster way there.
 constexpr int kWaveSteps = 64;
 constexpr int kPoolBudget = 64;
 constexpr int64_t kWaveMinRows = (int64_t)1 << 18;
+// The default split for the batch size.  With few solves left of each row, the
+// bulk of a batch of up to some millions of rows is soon done and the rest of
+// the lock-step launches wait for nothing: four steps, then the pool to the
+// end (ms at 64 / 64 and so, mean of five batches: vertex-face 270,000 rows 8.1
+// and 3.6, 1M 10.7 and 5.1, 4M 19.6 and 16.4; edge-edge 25.0 and 18.6, 27.1 and
+// 23.5, but 4M 39.1 and 42.7).  10M vertex-face rows: 33.6 at 64 / 64, 30.6
+// with sixteen steps and the pool.
+inline void default_split(int slots, int64_t rows, int &steps, int &budget) {
+  const bool vf = slots == 4;
+  if (!vf && rows >= (int64_t)1 << 21) return;
+  steps = rows < (int64_t)1 << 22 ? 4 : 16;
+  budget = 0;
+}
 // Job lists: one per (working phase, current degree 3..6).
 constexpr int kWaveBins = 16;
 
@@ -485,11 +498,12 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
   // than sc.pool_slots_min.  A small batch then spreads over more warps
   // instead of filling the first warps' slots while the rest of the grid
   // idles: each warp advances fewer solves per iteration, with fewer
-  // divergent paths, and so each of them more often.  The wavefront's
-  // leftovers (long solves, where packing lanes of one phase pays) fill
-  // every slot.
+  // divergent paths, and so each of them more often.  What a wavefront
+  // leaves for a limited number of further steps (long solves, where packing
+  // lanes of one phase pays) fills every slot.
   const int share = (int)(((int64_t)njobs + gridDim.x - 1) / gridDim.x);
-  const int lo = tail ? POOL : (sc.pool_slots_min < 1 ? 1 : sc.pool_slots_min);
+  const bool leftovers = tail && pj.budget > 0;
+  const int lo = leftovers ? POOL : (sc.pool_slots_min < 1 ? 1 : sc.pool_slots_min);
   const int lim = share < lo ? lo : (share < POOL ? share : POOL);
   auto state = [&](int k) {
     const int64_t g = job_of[k];
@@ -577,7 +591,7 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
       if (exhausted && !pending) break;
       continue;
     }
-    if (sc.pool_phase_sync && !tail) {
+    if (sc.pool_phase_sync && !leftovers) {
       // The phase of this moment (rotating every 2^k cycles of the SM's
       // clock, alike for the warps of one SM) when it holds at least half
       // as many solves as the most populated one: the SM's warps then run
@@ -1013,7 +1027,8 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
     }
     launch_next(stage_build<Polys>, build_grid, kStageThreads, 0, s, b, list, tile * sc.cap, sc, spread);
     if (sc.wd && sc.wave_steps > 0 && b.n >= sc.wave_min_rows) {
-      const int steps = sc.wave_steps;
+      int steps = sc.wave_steps, budget = sc.pool_budget;
+      if (steps == kWaveSteps && budget == kPoolBudget) default_split(Polys::kSlots, b.n, steps, budget);
       const int64_t lstride = (int64_t)kWaveBins * sc.jcap;
       // counts: 3 rotating sets, then the tail and spill lengths
       e = cudaMemsetAsync(sc.wcount, 0, (3 * kWaveBins + 2) * sizeof(unsigned), s);
@@ -1032,7 +1047,7 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
       // can be resident at once.  The wavefront lists are free again and hold
       // the spilled jobs.
       launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc,
-                  PoolJobs{sc.tail, tcount, sc.pool_budget, sc.wlist, scount});
+                  PoolJobs{sc.tail, tcount, budget, sc.wlist, scount});
       StageScratch last = sc;
       last.shift_after = sc.shift_after < 1 ? sc.shift_after : 1;
       launch_next(wave_finish<Polys>, num_sms * 32, 32, 0, s, last, sc.wlist, scount);

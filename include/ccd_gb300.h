@@ -96,7 +96,11 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *   "wave_steps"     root-solver steps taken in lock-step over all queued
  *                    polynomials of a large batch before the unfinished ones
  *                    continue in the per-warp pool solver (0: the pool
- *                    solver only); default 64, at most 4096
+ *                    solver only); default 64, at most 4096.  With this and
+ *                    pool_budget at their defaults the batch size decides:
+ *                    4 steps and no budget below 2^22 vertex-face or 2^21
+ *                    edge-edge rows, 16 and no budget for larger
+ *                    vertex-face batches
  *   "wave_min_rows"  smallest batch (rows) that uses those lock-step steps;
  *                    default 262144
  *   "count_slab_tests" 1: the broad phase counts its traversal's slab tests
