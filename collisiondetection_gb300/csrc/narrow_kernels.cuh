@@ -108,8 +108,6 @@ __global__ void __launch_bounds__(kThreads) prims_fp64_list_kernel(PrimBatch b, 
 // compacted into `list` with one atomic per warp (ballot + popc prefix).
 template <int KIND>
 __global__ void __launch_bounds__(kThreads) prims_cull_kernel(PrimBatch b, int32_t *__restrict__ list) {
-  // The first stage of the refinement may be launched; it waits for the list.
-  cudaTriggerProgrammaticLaunchCompletion();
   const unsigned lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
