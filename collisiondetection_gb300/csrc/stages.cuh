@@ -599,6 +599,13 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
       if (exhausted && !pending) break;
       continue;
     }
+    // A warp whose slots are all taken does not ask for jobs, so with one slot
+    // to fill it looks whether any are left: its only solve may be its last.
+    if (!exhausted && working == 1 && lim == 1) {
+      unsigned next = 0;
+      if (lane == 0) next = *(volatile unsigned *)&sc.queue[kMaxSlots];
+      exhausted = __shfl_sync(0xffffffffu, next, 0) >= (unsigned)njobs;
+    }
     if (sc.pool_phase_sync && !leftovers) {
       // The phase of this moment (rotating every 2^k cycles of the SM's
       // clock, alike for the warps of one SM) when it holds at least half
