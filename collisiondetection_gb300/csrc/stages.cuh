@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
     const int64_t r = w + lane;
     bool active = (int)lane < per && r < end;
     const int rows = end - w < per ? (int)(end - w) : per;
-    double x[24];
+    double x[24], dist[7];  // dist: the distance sextic, kept for the queue
     double eta = 0.0;
     int64_t i = 0;
     bool bounded = false;
@@ -338,20 +338,24 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
       for (int j = 0; j < 24; j++) x[j] = __ldg(src + j);
       eta = b.eta_per_row ? __ldg(b.eta + i) : __ldg(b.eta);
       bounded = sc.classify;
+      // The distance sextic first: a row whose sextic cannot be bounded (its
+      // leading coefficient vanishes when one feature is still) is left to the
+      // solver, and its sides need no look here.
 #pragma unroll 1
-      for (int slot = 0; slot < K; slot++) {
-        if (!sc.classify && slot != kDist) continue;
-        double op[7];
+      for (int k = 0; k < K && (k == 0 || bounded); k++) {
+        const int slot = k == 0 ? kDist : (k <= kDist ? k - 1 : k);
+        double side[7];
+        double *op = k == 0 ? dist : side;
         Polys::coeffs(x, eta, slot, op);
         if (slot == kDist) {
           double m = 0.0;
 #pragma unroll
-          for (int k = 0; k <= 6; k++) m = smax(m, fabs(op[k]));
+          for (int c = 0; c <= 6; c++) m = smax(m, fabs(op[c]));
           if (fabs(op[5]) + fabs(op[6]) <= kDeferTail * m) {
             unsolved = 1u << (kUnsolvedShift + kDist);
             bool other = false;
 #pragma unroll
-            for (int k = 1; k < 6; k++) other = other || op[k] != 0.0;
+            for (int c = 1; c < 6; c++) other = other || op[c] != 0.0;
             if (op[6] == 0.0 && op[0] != 0.0 && other) unsolved |= kZeroAtStart;
           }
         }
@@ -388,9 +392,10 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
 #pragma unroll 1
     for (int slot = 0; slot < K; slot++) {
       const bool solve = active && !((unsolved >> (kUnsolvedShift + slot)) & 1u);
-      double op[7];
+      double side[7];
+      double *op = slot == kDist ? dist : side;
       if (solve) {
-        Polys::coeffs(x, eta, slot, op);
+        if (slot != kDist) Polys::coeffs(x, eta, slot, op);
       } else if (active && slot != kDist) {
         SpanList sl;
         cls::stand_in(need.near, sl);

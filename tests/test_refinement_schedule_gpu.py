@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 import collisiondetection_gb300 as C
+from collisiondetection_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,17 @@ def test_small_flat_batch_finishes_its_last_solves_together(kind):
         np.testing.assert_array_equal(h, h64)
         np.testing.assert_array_equal(t[h64 == 1].view(np.uint64), t64[h64 == 1].view(np.uint64))
     assert one <= 2.0 * four
+
+
+@pytest.mark.parametrize("kind", [C.VERTEX_FACE, C.EDGE_EDGE])
+@pytest.mark.parametrize("n", [1, 33, 5000])
+def test_still_rows_equal_fp64_kernel(ctx, kind, n):
+    # Sextics whose leading coefficient vanishes beside ordinary ones in the
+    # same warp: the sextic formed once serves the bounds and the queue.
+    rows = _still(n)
+    rows[::3] = W.primitive_batch(kind, n, seed=13)[::3]
+    h64, t64 = ctx.prim_batch(kind, rows, 1e-3, path=C.PATH_FP64)
+    for path in (C.PATH_CULL_REFINE, C.PATH_REFINE_ALL):
+        h, t = ctx.prim_batch(kind, rows, 1e-3, path=path)
+        np.testing.assert_array_equal(h, h64)
+        np.testing.assert_array_equal(t[h64 == 1].view(np.uint64), t64[h64 == 1].view(np.uint64))
