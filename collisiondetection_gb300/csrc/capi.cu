@@ -28,7 +28,7 @@ int ensure_stage(ccd_context *ctx, StageBuf &sb, int64_t rows, cudaStream_t s) {
   int64_t cap = std::min<int64_t>(std::max<int64_t>(rows, 1), kStageTileRows);
   // The wavefront solver's scratch (about 3 KB per row) only for batches
   // large enough to use it.
-  const bool wave = ctx->opt_wave_steps > 0 && rows >= ctx->opt_wave_min_rows;
+  const bool wave = ctx->opt_wave_steps != 0 && rows >= ctx->opt_wave_min_rows;
   if (sb.cap >= cap && (sb.view.wd != nullptr || !wave)) return CCD_OK;
   cap = std::max<int64_t>(cap, sb.cap);
   CCD_CUDA(cudaStreamSynchronize(s));
@@ -121,7 +121,8 @@ static ccd::StageScratch stage_view(const ccd_context *ctx, const StageBuf &stag
   view.wave_min_rows = ctx->opt_wave_min_rows;
   view.pool_budget = ctx->opt_pool_budget;
   view.warp_finish = ctx->opt_warp_finish;
-  view.shift_after = ctx->opt_shift_after;
+  view.shift_after = ctx->opt_shift_after < 0 ? ccd::kShiftAfter : ctx->opt_shift_after;
+  view.finish_shift_after = ctx->opt_shift_after < 0 ? ccd::kFinishShiftAfter : ctx->opt_shift_after;
   view.pool_slots = ctx->opt_pool_slots;
   view.pool_slots_min = ctx->opt_pool_slots_min;
   view.pool_all = ctx->opt_pool_all;

@@ -176,13 +176,16 @@ int ccd_autotune_prim_batch(ccd_context *ctx, int kind, int64_t n, const double 
   const int64_t saved_min_rows = saved.min_rows;
   ctx->profiling = false;
 
-  // The context's own settings come first: their output is the one every
-  // other candidate must reproduce.  Then the pool kernel alone, then the
+  // The context's own settings come first, with the steps and budget that they
+  // give this batch: their output is the one every other candidate must
+  // reproduce.  Then the pool kernel alone, then the
   // wavefront at each step count with each pool budget, then short pool
   // budgets whose leftovers finish one per warp with their stages' remaining
   // shifts tried at once.
   std::vector<Split> cands;
-  cands.push_back({n >= saved_min_rows ? saved_steps : 0, saved_budget, saved_finish, saved_after});
+  int own_steps = saved_steps, own_budget = saved_budget;
+  ccd::resolve_split(kind == CCD_VERTEX_FACE, n, own_steps, own_budget);
+  cands.push_back({n >= saved_min_rows ? own_steps : 0, own_budget, saved_finish, saved_after});
   cands.push_back({0, 0, saved_finish, saved_after});
   for (int steps : {16, 32, 48, 64, 96, 128})
     for (int budget : {0, 256, 4096}) cands.push_back({steps, budget, saved_finish, saved_after});
@@ -280,7 +283,17 @@ int ccd_autotune_prim_batch(ccd_context *ctx, int kind, int64_t n, const double 
 
   out->best_ms = best_ms;
   saved.committed = true;
-  if (best.wave_steps > 0) {
+  out->wave_steps = best.wave_steps;
+  out->pool_budget = best.pool_budget;
+  if (best_i == 0) {
+    // The context's own split: its options stay as they were (those that were
+    // not set go on following the batch size).
+    ctx->opt_wave_steps = saved_steps;
+    ctx->opt_pool_budget = saved_budget;
+    ctx->opt_warp_finish = saved_finish;
+    ctx->opt_shift_after = saved_after;
+    ctx->opt_wave_min_rows = saved_min_rows;
+  } else if (best.wave_steps > 0) {
     // Batches as large as this one take the wavefront with the chosen split.
     ctx->opt_wave_steps = best.wave_steps;
     ctx->opt_pool_budget = best.pool_budget;
@@ -296,10 +309,12 @@ int ccd_autotune_prim_batch(ccd_context *ctx, int kind, int64_t n, const double 
     ctx->opt_shift_after = saved_after;
     ctx->opt_wave_min_rows = std::max<int64_t>(saved_min_rows, n + 1);
   }
-  out->wave_steps = ctx->opt_wave_steps;
-  out->pool_budget = ctx->opt_pool_budget;
+  if (best.wave_steps == 0) {  // the split of the larger batches
+    out->wave_steps = own_steps;
+    out->pool_budget = own_budget;
+  }
   out->warp_finish = ctx->opt_warp_finish;
-  out->shift_after = ctx->opt_shift_after;
+  out->shift_after = ctx->opt_shift_after < 0 ? ccd::kFinishShiftAfter : ctx->opt_shift_after;
   out->wave_min_rows = ctx->opt_wave_min_rows;
   out->chosen = best_i;
   return CCD_OK;

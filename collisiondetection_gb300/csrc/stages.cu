@@ -45,7 +45,8 @@ StageScratch stage_scratch_view(void *base, int64_t cap) {
   sc.wave_min_rows = 0;
   sc.pool_budget = 0;
   sc.warp_finish = 1;
-  sc.shift_after = 2;
+  sc.shift_after = kShiftAfter;
+  sc.finish_shift_after = kFinishShiftAfter;
   sc.pool_slots = stages::kWarpPool;
   sc.pool_slots_min = stages::kWarpPool;
   sc.pool_all = 0;
@@ -73,9 +74,9 @@ void attach_wave(StageScratch &sc, void *base) {
   sc.wcount = (unsigned *)p;
   p += up((3 * kWaveBins + 2) * sizeof(unsigned));
   sc.tail = (uint32_t *)p;
-  sc.wave_steps = kWaveSteps;
+  sc.wave_steps = kBySize;
   sc.wave_min_rows = kWaveMinRows;
-  sc.pool_budget = kPoolBudget;
+  sc.pool_budget = kBySize;
 }
 
 namespace {

@@ -61,19 +61,24 @@ constexpr int kStageThreads = 128;
 constexpr int kWaveSteps = 64;
 constexpr int kPoolBudget = 64;
 constexpr int64_t kWaveMinRows = (int64_t)1 << 18;
-// The default split for the batch size.  With few solves left of each row, the
-// bulk of a batch of up to some millions of rows is soon done and the rest of
-// the lock-step launches wait for nothing: four steps, then the pool to the
-// end (ms at 64 / 64 and so, mean of five batches: vertex-face 270,000 rows 8.1
-// and 3.6, 1M 10.7 and 5.1, 4M 19.6 and 16.4; edge-edge 25.0 and 18.6, 27.1 and
-// 23.5, but 4M 39.1 and 42.7).  10M vertex-face rows: 33.6 at 64 / 64, 30.6
-// with sixteen steps and the pool.
-inline void default_split(int slots, int64_t rows, int &steps, int &budget) {
-  const bool vf = slots == 4;
-  if (!vf && rows >= (int64_t)1 << 21) return;
-  steps = rows < (int64_t)1 << 22 ? 4 : 16;
-  budget = 0;
+// Steps and budget that nobody has set are kBySize: the batch size decides.
+// With few solves left of each row, the bulk of a batch of up to some millions
+// of rows is soon done and the rest of the lock-step launches wait for nothing:
+// four steps, then the pool to the end (ms at 64 / 64 and so, mean of five
+// batches: vertex-face 270,000 rows 8.1 and 3.6, 1M 10.7 and 5.1, 4M 19.6 and
+// 16.4; edge-edge 25.0 and 18.6, 27.1 and 23.5, but 4M 39.1 and 42.7).  10M
+// vertex-face rows: 33.6 at 64 / 64, 30.6 with sixteen steps and the pool.
+// A budget that is set goes with the full number of steps: after four, too much
+// would be left for the one-per-warp finish.
+constexpr int kBySize = -1;
+inline void resolve_split(bool vf, int64_t rows, int &steps, int &budget) {
+  const bool brief = vf || rows < (int64_t)1 << 21;
+  if (steps == kBySize) steps = !brief || budget != kBySize ? kWaveSteps : (rows < (int64_t)1 << 22 ? 4 : 16);
+  if (budget == kBySize) budget = brief ? 0 : kPoolBudget;
 }
+// Failed shifts before a stage's remaining ones run at once: in the pool, and
+// in the one-per-warp finish, whose solves have failed some already.
+constexpr int kShiftAfter = 2, kFinishShiftAfter = 1;
 // Job lists: one per (working phase, current degree 3..6).
 constexpr int kWaveBins = 16;
 
@@ -102,13 +107,13 @@ struct StageScratch {
   uint32_t *wlist;      // [2][bin < 16][jcap]           jobs per (phase, degree)
   unsigned *wcount;     // [3][16] list lengths (rotating), then the tail and spill lengths
   uint32_t *tail;       // [jcap]                        jobs left after the wavefront steps
-  int wave_steps;       // wavefront steps (0: pool kernel only)
+  int wave_steps;       // wavefront steps (0: pool kernel only; kBySize)
   int64_t wave_min_rows;
   int pool_budget;      // steps the pool kernel gives a resumed job before handing it on
   int warp_finish;      // how the last solves run: 0 on one lane; 1 on all 32 lanes of their warp
                         // (ccd_jt_warp.h); 2 with a stage's remaining shifts tried at once, one per
                         // lane (ccd_jt_shifts.h), once shift_after of its shifts have failed
-  int shift_after;
+  int shift_after, finish_shift_after;  // in the pool, and in the one-per-warp finish
   int pool_slots;       // pool kernel of a batch the wavefront does not take: 32 or 64 slots per warp
   int pool_slots_min;   // pool kernel: fewest slots a warp may fill (its share of a small batch is spread)
   int pool_all;         // pool kernel: once the queue is drained, at most this many solves left step together
@@ -1046,9 +1051,9 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
       if (e != cudaSuccess) return e;
     }
     launch_next(stage_build<Polys>, build_grid, kStageThreads, 0, s, b, list, tile * sc.cap, sc, spread);
-    if (sc.wd && sc.wave_steps > 0 && b.n >= sc.wave_min_rows) {
+    if (sc.wd && sc.wave_steps != 0 && b.n >= sc.wave_min_rows) {
       int steps = sc.wave_steps, budget = sc.pool_budget;
-      if (steps == kWaveSteps && budget == kPoolBudget) default_split(Polys::kSlots, b.n, steps, budget);
+      resolve_split(Polys::kSlots == 4, b.n, steps, budget);
       const int64_t lstride = (int64_t)kWaveBins * sc.jcap;
       // counts: 3 rotating sets, then the tail and spill lengths
       e = cudaMemsetAsync(sc.wcount, 0, (3 * kWaveBins + 2) * sizeof(unsigned), s);
@@ -1069,7 +1074,7 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
       launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc,
                   PoolJobs{sc.tail, tcount, budget, sc.wlist, scount});
       StageScratch last = sc;
-      last.shift_after = sc.shift_after < 1 ? sc.shift_after : 1;
+      last.shift_after = sc.finish_shift_after;
       launch_next(wave_finish<Polys>, num_sms * 32, 32, 0, s, last, sc.wlist, scount);
       *launches += steps + 4;
     } else {

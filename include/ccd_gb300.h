@@ -96,11 +96,11 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *   "wave_steps"     root-solver steps taken in lock-step over all queued
  *                    polynomials of a large batch before the unfinished ones
  *                    continue in the per-warp pool solver (0: the pool
- *                    solver only); default 64, at most 4096.  With this and
- *                    pool_budget at their defaults the batch size decides:
- *                    4 steps and no budget below 2^22 vertex-face or 2^21
- *                    edge-edge rows, 16 and no budget for larger
- *                    vertex-face batches
+ *                    solver only); at most 4096.  Where this is not set the
+ *                    batch size decides: 4 steps below 2^22 vertex-face or
+ *                    2^21 edge-edge rows, 16 for larger vertex-face and 64
+ *                    for larger edge-edge batches (64 for all where only
+ *                    pool_budget is set)
  *   "wave_min_rows"  smallest batch (rows) that uses those lock-step steps;
  *                    default 262144
  *   "count_slab_tests" 1: the broad phase counts its traversal's slab tests
@@ -122,7 +122,9 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *                    smaller register budget; default 3
  *   "pool_budget"    further steps the unfinished polynomials get, many per
  *                    warp, before the last ones are finished one per warp
- *                    (0: no limit); default 64
+ *                    (0: no limit).  Where this is not set: 64 for
+ *                    edge-edge batches of 2^21 rows or more, no limit for
+ *                    the others
  *   "pool_slots"     pool solver of a batch the wavefront does not take:
  *                    solver slots per warp, 64 (five warps per SM) or 32
  *                    (ten warps per SM); default 64
@@ -149,8 +151,8 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *                    remaining shifts, the first that converges kept (the
  *                    same results as the sequential order); default 2
  *   "shift_after"    warp_finish 2: shifts of a stage tried one at a time
- *                    before the remaining ones run at once (at most 1 by the
- *                    one-per-warp finish); in [0, 19], default 2
+ *                    before the remaining ones run at once; in [0, 19],
+ *                    default 2, and 1 by the one-per-warp finish
  *   "chunk_rows"     ccd_prim_batch: largest chunk (rows) streamed through
  *                    the device, two in flight; a batch is cut into equal
  *                    chunks; in [1024, 2^26], default 2^23
@@ -255,11 +257,12 @@ int ccd_fp64_peak(ccd_context *ctx, int reps, ccd_fp64_peak_result *out);
  * remaining shifts tried at once, and the context's own split once
  * more, checks that every split's hits and contact times equal the first
  * split's bit for bit, and sets the fastest matching split as the context's
- * options.  Blocks until done;
+ * options (which stay as they were where its own split is the fastest).
+ * Blocks until done;
  * allocates its own output buffers.  Results of later batches never change,
  * only their speed. */
 typedef struct {
-  int32_t wave_steps;    /* the context's options after the call */
+  int32_t wave_steps;    /* the split that such a batch takes after the call, from wave_min_rows on */
   int32_t pool_budget;
   int64_t wave_min_rows;
   int32_t candidates;    /* splits timed */
