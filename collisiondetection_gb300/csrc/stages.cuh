@@ -98,7 +98,7 @@ struct StageScratch {
   int32_t *row_id;      // [cap]                batch row of each tile row
   int32_t *redo;        // [cap]                tile rows of the second round
   double *roots;        // [slot][k < 6][cap]   roots found by the solver
-  bool classify;        // drop polynomials whose list is not needed (ccd_classify.h)
+  bool classify;        // leave out polynomials whose list is not needed (ccd_classify.h); false: solve all
   // Wavefront solver (null when not attached: the pool kernel then solves
   // every queued polynomial).  Jobs are numbered slot by slot (queue order).
   int64_t jcap;         // kMaxSlots * cap
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
       // leading coefficient vanishes when one feature is still) is left to the
       // solver, and its sides need no look here.
 #pragma unroll 1
-      for (int k = 0; k < K && (k == 0 || bounded); k++) {
+      for (int k = 0; k < K && bounded; k++) {
         const int slot = k == 0 ? kDist : (k <= kDist ? k - 1 : k);
         double side[7];
         double *op = k == 0 ? dist : side;
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
             if (op[6] == 0.0 && op[0] != 0.0 && other) unsolved |= kZeroAtStart;
           }
         }
-        if (sc.classify) bounded = R::put(mine + lane * kStride, slot, op) && bounded;
+        bounded = R::put(mine + lane * kStride, slot, op);
       }
     }
     __syncwarp();
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
       double side[7];
       double *op = slot == kDist ? dist : side;
       if (solve) {
-        if (slot != kDist) Polys::coeffs(x, eta, slot, op);
+        if (slot != kDist || !sc.classify) Polys::coeffs(x, eta, slot, op);
       } else if (active && slot != kDist) {
         SpanList sl;
         cls::stand_in(need.near, sl);
@@ -1085,12 +1085,14 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
       *launches += 1;
     }
     launch_next(stage_combine<Polys, true>, grid, kStageThreads, 0, s, b, sc);
+    *launches += 2;
+    if (!sc.classify) continue;
     // Second round: usually few rows or none, so the pool kernel alone.
     StageScratch sc2 = sc;
     sc2.queue = sc.queue + kQueueRound;
     launch_next(stage_roots<Polys, kWarpPool>, pool_grid, 32, kPoolSmem, s, sc2, queued);
     launch_next(stage_combine<Polys, false>, grid, kStageThreads, 0, s, b, sc);
-    *launches += 4;
+    *launches += 2;
   }
   return cudaGetLastError();
 }

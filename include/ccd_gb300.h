@@ -46,14 +46,16 @@ typedef enum {
   /* FP64 evaluation of every row, op-for-op with the reference. */
   CCD_PATH_FP64 = 0,
   /* Outward-bounded FP32 rejection of rows whose result is provably "no
-   * hit", then the FP64 evaluation of the surviving rows only.  Same results
-   * as CCD_PATH_FP64 (the FP32 stage never rejects a row that hits).
+   * hit", then the FP64 evaluation of the surviving rows only; of
+   * vertex-face and edge-edge rows, only the polynomials that their signs
+   * leave undecided are solved.  Same results as CCD_PATH_FP64 (the FP32
+   * stage never rejects a row that hits).
    * Vertex-vertex rows (one quadratic) are always evaluated in FP64. */
   CCD_PATH_CULL_REFINE = 1,
-  /* No FP32 stage: every row through the FP64 refinement that
-   * CCD_PATH_CULL_REFINE applies to its survivors (batched root solvers for
-   * vertex-face and edge-edge rows).  Same results; the all-FP64 baseline
-   * that isolates what the FP32 stage saves. */
+  /* No FP32 stage and nothing decided from signs: every row, and every
+   * polynomial of it, through the batched FP64 root solvers that
+   * CCD_PATH_CULL_REFINE applies to what it leaves of its survivors.  Same
+   * results; the all-FP64 baseline. */
   CCD_PATH_REFINE_ALL = 2
 } ccd_path;
 
