@@ -256,16 +256,6 @@ __device__ __forceinline__ void queue_slot(const StageScratch &sc, int slot, int
   }
 }
 
-// A distance sextic whose last two coefficients are this small beside the
-// largest has roots at (or within rounding of) t = 0: features that start in
-// contact with their common plane, as the edges of a flat sheet do.  Such a
-// solve can run through all 20 shifts (some 13,000 steps, against about 20
-// for others), and the row's other lists usually share no time beyond 0, so
-// it waits for them (stage_combine).  On a flat sheet in rigid motion with
-// jitter, 86% of the solver steps of these sextics are saved.
-// (24 meshes, sheets among them: 465 -> 202 ms with it and the classification.)
-constexpr double kDeferTail = 1e-9;
-
 // The decision of ccd_classify.h for one row by a warp; w: the row's words.
 template <class Polys>
 __device__ __forceinline__ cls::Need classify_row(const float *w) {
@@ -353,16 +343,9 @@ __global__ void __launch_bounds__(kStageThreads) stage_build(PrimBatch b, const 
         double *op = k == 0 ? dist : side;
         Polys::coeffs(x, eta, slot, op);
         if (slot == kDist) {
-          double m = 0.0;
-#pragma unroll
-          for (int c = 0; c <= 6; c++) m = smax(m, fabs(op[c]));
-          if (fabs(op[5]) + fabs(op[6]) <= kDeferTail * m) {
-            unsolved = 1u << (kUnsolvedShift + kDist);
-            bool other = false;
-#pragma unroll
-            for (int c = 1; c < 6; c++) other = other || op[c] != 0.0;
-            if (op[6] == 0.0 && op[0] != 0.0 && other) unsolved |= kZeroAtStart;
-          }
+          const unsigned wait = cls::waits(op);
+          if (wait & cls::kWaits) unsolved = 1u << (kUnsolvedShift + kDist);
+          if (wait & cls::kZeroAtStart) unsolved |= kZeroAtStart;
         }
         bounded = R::put(mine + lane * kStride, slot, op);
       }
@@ -885,37 +868,9 @@ __global__ void __launch_bounds__(32) wave_finish(StageScratch sc, const uint32_
   }
 }
 
-// Whether the side lists of a row (every list but the distance's) share a
-// time; beyond: one after t = 0.
-template <int N>
-__device__ __forceinline__ bool sides_meet(const SpanList *l, bool &beyond) {
-  bool meets = false;
-  beyond = false;
-  for (int i = 0; i < l[0].n; i++)
-    for (int j = 0; j < l[1].n; j++) {
-      const double lo1 = smax(l[0].s[i].l, l[1].s[j].l), hi1 = smin(l[0].s[i].u, l[1].s[j].u);
-      if (lo1 > hi1) continue;
-      for (int k = 0; k < l[2].n; k++) {
-        const double lo2 = smax(lo1, l[2].s[k].l), hi2 = smin(hi1, l[2].s[k].u);
-        if (lo2 > hi2) continue;
-        for (int m = 0; m < (N == 4 ? l[N - 1].n : 1); m++) {
-          const double lo = N == 4 ? smax(lo2, l[N - 1].s[m].l) : lo2, hi = N == 4 ? smin(hi2, l[N - 1].s[m].u) : hi2;
-          if (lo > hi) continue;
-          meets = true;
-          if (hi > 0.0) beyond = true;
-        }
-      }
-    }
-  return meets;
-}
-
 // The decision of each kept row.  First round: a row with unsolved slots is
 // decided if what is solved settles it, and goes to the second round if not:
-//   * unsolved distance sextic: the row misses when its side lists share no
-//     time.  Where they share t = 0 alone, the sextic vanishes there exactly
-//     and the edges are parallel there, the sextic's list holds the span
-//     [0, 0], which counts as parallel and rules out every combination that
-//     touches it: the row misses too;
+//   * unsolved distance sextic: cls::settled_without_sextic;
 //   * unsolved sides of an edge-edge row: their replacement holds as long as
 //     no span is parallel (the parallel rule looks at single combinations of
 //     spans).
@@ -952,28 +907,19 @@ __global__ void __launch_bounds__(kStageThreads) stage_combine(PrimBatch b, Stag
       double t = 0.0;
       bool h = false;
       if constexpr (K == 4) {
-        if (unsolved >> kDist & 1u) {
-          bool beyond;
-          again = sides_meet<3>(l, beyond);
-        } else {
+        if (unsolved >> kDist & 1u)
+          again = !cls::settled_without_sextic<4>(nullptr, l, false);
+        else
           h = vf_combine(l[0], l[1], l[2], l[3], t);
-        }
       } else {
         double x[24];
         const double *src = b.rows + i * 24;
 #pragma unroll
         for (int j = 0; j < 24; j++) x[j] = __ldg(src + j);
-        SpanList cop, par;
         if (unsolved >> kDist & 1u) {
-          bool beyond;
-          again = sides_meet<4>(l + 1, beyond);
-          if (again && !beyond && (word & kZeroAtStart)) {
-            l[0].n = 1;
-            l[0].s[0] = Span{0.0, 0.0};
-            ee_split_parallel(x, l[0], cop, par);
-            again = par.n == 0;
-          }
+          again = !cls::settled_without_sextic<5>(x, l, (word & kZeroAtStart) != 0);
         } else {
+          SpanList cop, par;
           ee_split_parallel(x, l[0], cop, par);
           again = unsolved && par.n > 0;
           if (!again) h = ee_combine(cop, par, l[1], l[2], l[3], l[4], t);
