@@ -229,10 +229,14 @@ constexpr unsigned kZeroAtStart = 2;  // and vanishes exactly at t = 0 beside ot
 
 // What distance sextic op (reference order) is, in these bits.
 CCD_HD unsigned waits(const double *op) {
-  double m = 0.0;
+  double m = 0.0, sum = 0.0;
 CCD_UNROLL
-  for (int c = 0; c <= 6; c++) m = smax(m, fabs(op[c]));
-  if (!(fabs(op[5]) + fabs(op[6]) <= kWaitTail * m)) return 0;
+  for (int c = 0; c <= 6; c++) {
+    m = smax(m, fabs(op[c]));
+    sum += fabs(op[c]);
+  }
+  // not one that is infinite or NaN: the solver reports it in the row's status
+  if (!(sum < 1e300) || !(fabs(op[5]) + fabs(op[6]) <= kWaitTail * m)) return 0;
   bool other = false;
 CCD_UNROLL
   for (int c = 1; c < 6; c++) other = other || op[c] != 0.0;

@@ -76,3 +76,14 @@ def test_which_sextics_wait():
     out = np.zeros(len(ops), np.uint8)
     _lib().hc_waits(ctypes.c_int64(len(ops)), ops.ctypes.data_as(P), out.ctypes.data_as(P))
     assert out.tolist() == [0, 1, 3, 1, 1]
+
+
+@pytest.mark.parametrize("at", range(7))
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_sextics_that_are_not_finite_do_not_wait(at, bad):
+    # the solver reports them in the row's status
+    op = np.array([[1.0, 2.0, 3.0, 4.0, 5.0, 0.0, 0.0]])
+    op[0, at] = bad
+    out = np.zeros(1, np.uint8)
+    _lib().hc_waits(ctypes.c_int64(1), op.ctypes.data_as(P), out.ctypes.data_as(P))
+    assert out[0] == 0
