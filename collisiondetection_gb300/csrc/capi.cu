@@ -508,18 +508,11 @@ int ccd_prim_batch(ccd_context *ctx, int kind, int path, int64_t n, const double
   return CCD_OK;
 }
 
-// One query.  A vertex-face or edge-edge row takes the staged refinement, whose
-// pool solves the row's polynomials on different warps; the FP64 kernel solves
-// them one after another on a lone lane.  Turning features that meet (us, the
-// slowest of four): vertex-face 398 there and 306 here, edge-edge 664 and 318.
-// A vertex-edge row has one quartic: 124 there, 142 here.
 static int single(ccd_context *ctx, int kind, const double *points, double eta, int *hit, double *t) {
   if (!ctx || !points || !hit || !t) return fail(ctx, CCD_ERR_INVALID_ARGUMENT, "null argument");
   uint8_t h = 0;
   double tt = *t;
-  const int path =
-      kind == CCD_VERTEX_FACE || kind == CCD_EDGE_EDGE ? CCD_PATH_CULL_REFINE : CCD_PATH_FP64;
-  int rc = ccd_prim_batch(ctx, kind, path, 1, points, &eta, 1, &h, &tt);
+  int rc = ccd_prim_batch(ctx, kind, CCD_PATH_FP64, 1, points, &eta, 1, &h, &tt);
   if (rc) return rc;
   *hit = h;
   if (h) *t = tt;

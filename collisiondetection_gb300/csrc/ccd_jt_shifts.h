@@ -72,17 +72,19 @@ __device__ __forceinline__ void take(LocalStorage &st, int src) {
 }
 
 // Runs the solve held (identically) by every lane of the warp to its end;
-// every lane returns with the final state.  All 32 lanes must call it.  A
+// every lane returns true with the final state, or false once *stop (where
+// there is one) is set.  All 32 lanes must call it.  A
 // stage's first `after` shifts run one at a time, every lane stepping the
 // same state (most stages end within them, and trying later shifts early
 // would only add divergent work); once `after` shifts of the stage have
 // failed, the remaining ones run at once.
-__device__ __noinline__ inline void run(LocalStorage &st, int after) {
+__device__ __noinline__ inline bool run(LocalStorage &st, int after, const volatile int *stop = nullptr) {
   const LocalState s{&st};
   const int lane = (int)(threadIdx.x & 31);
   for (;;) {
     const int mode = s.I(MODE);
-    if (mode == kDone) return;
+    if (mode == kDone) return true;
+    if (stop && __any_sync(kFull, *stop != 0)) return false;
     if (mode == kInit) {
       step_init(s);
       continue;
@@ -98,6 +100,7 @@ __device__ __noinline__ inline void run(LocalStorage &st, int after) {
     if (lane > 0 && running) start_later_shift(s, lane);
     int w;
     for (;;) {
+      if (stop && __any_sync(kFull, *stop != 0)) return false;
       if (running) {
         step(s);
         const int o = shift_outcome(s, c, n0);

@@ -3,6 +3,7 @@
 
 namespace ccd {
 
+cudaError_t launch_query(const PrimBatch &, cudaStream_t);
 cudaError_t launch_vf_fp64(const PrimBatch &, int, cudaStream_t);
 cudaError_t launch_ee_fp64(const PrimBatch &, int, cudaStream_t);
 cudaError_t launch_ve_fp64(const PrimBatch &, int, cudaStream_t);
@@ -14,6 +15,7 @@ cudaError_t launch_ve_fp64_list(const PrimBatch &, const int32_t *, int, cudaStr
 
 cudaError_t launch_prims_fp64(const PrimBatch &b, int num_sms, cudaStream_t s) {
   if (b.n <= 0) return cudaSuccess;
+  if (b.n == 1 && b.kind <= 1) return launch_query(b, s);
   switch (b.kind) {
     case 0: return launch_vf_fp64(b, num_sms, s);
     case 1: return launch_ee_fp64(b, num_sms, s);
