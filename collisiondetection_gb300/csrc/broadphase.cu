@@ -64,8 +64,30 @@ inline unsigned grid_of(int64_t n) { return (unsigned)std::max<int64_t>(1, (n + 
 // face needs comparisons only.  The FP64 pipe bounds this stage, and a vertex
 // of a closed mesh or a sheet lies in six faces: its projections are formed
 // once instead of six times.  211,970 faces over 106,498 vertices: 336 us with
-// the projections formed per face, now 63 us (vertices) + 48 us (faces).
+// the projections formed per face, now 57 us (vertices) + 53 us (faces).
+//
+// A face's bounds run over the entries of its vertices in order, and a NaN
+// among them drops what came before it (std::min returns its first argument
+// when the comparison fails).  Bounds of a vertex cannot say that of the face's
+// earlier vertices, so a vertex with a NaN is marked by a lower bound above the
+// upper one and its entries are taken one by one.
 constexpr int kVertexSlab = 26;
+
+// Entry e of vertex v: of the two of a step, or of a multi-entry history's
+// (src/KDOPBroadPhase.cpp:60-70).
+__device__ __forceinline__ const double *entry_pos(const BroadphaseParams &p, int v, int e) {
+  return p.hoff ? p.hpos + 3 * (int64_t)e : (e ? p.qe : p.qs) + 3 * (int64_t)v;
+}
+
+// KDOPBroadPhase.cpp:66-67 (pos . axis) / AABBBroadPhase.cpp:38-39 (pos[k])
+template <int K>
+__device__ __forceinline__ double project(const double *pos, const Axes &ax, int k) {
+  return K == 13 ? (pos[0] * ax.a[k][0] + pos[1] * ax.a[k][1]) + pos[2] * ax.a[k][2] : pos[k < 3 ? k : 0];
+}
+
+// Whether the result of an FP64 operation is NaN (a quiet one), on the integer
+// pipe.
+__device__ __forceinline__ bool is_nan(double x) { return (__double2hiint(x) & 0x7fffffff) > 0x7ff00000; }
 
 __global__ void __launch_bounds__(kThreads) vertex_slabs(int nv, BroadphaseParams p, Axes ax, double *out) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,18 +98,22 @@ __global__ void __launch_bounds__(kThreads) vertex_slabs(int nv, BroadphaseParam
     lo[k] = INFINITY;
     hi[k] = -INFINITY;
   }
-  // every History entry of the vertex (src/KDOPBroadPhase.cpp:60-70): the two
-  // of a step, or the entries of a multi-entry history
+  bool nan = false;
   const int e0 = p.hoff ? p.hoff[v] : 0, e1 = p.hoff ? p.hoff[v + 1] : 2;
   for (int e = e0; e < e1; e++) {
-    const double *pos = p.hoff ? p.hpos + 3 * (int64_t)e : (e ? p.qe : p.qs) + 3 * (int64_t)v;
-    const double px = pos[0], py = pos[1], pz = pos[2];
+    const double *src = entry_pos(p, v, e);
+    const double pos[3] = {src[0], src[1], src[2]};
 #pragma unroll
     for (int k = 0; k < 13; k++) {
-      const double val = (px * ax.a[k][0] + py * ax.a[k][1]) + pz * ax.a[k][2];  // KDOPBroadPhase.cpp:66-67
-      lo[k] = smin(val - p.eta, lo[k]);
-      hi[k] = smax(val + p.eta, hi[k]);
+      const double val = project<13>(pos, ax, k), below = val - p.eta, above = val + p.eta;
+      nan = nan || is_nan(below) || is_nan(above);
+      lo[k] = smin(below, lo[k]);
+      hi[k] = smax(above, hi[k]);
     }
+  }
+  if (nan) {
+    lo[0] = INFINITY;
+    hi[0] = -INFINITY;
   }
   double2 *q = reinterpret_cast<double2 *>(out + (int64_t)kVertexSlab * v);
 #pragma unroll
@@ -95,22 +121,54 @@ __global__ void __launch_bounds__(kThreads) vertex_slabs(int nv, BroadphaseParam
     q[k] = make_double2(2 * k < 13 ? lo[2 * k] : hi[2 * k - 13], 2 * k + 1 < 13 ? lo[2 * k + 1] : hi[2 * k + 1 - 13]);
 }
 
+// Bounds of face f over the entries of its vertices, in order.
 template <int K>
-__global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, BroadphaseParams p, const double *vslab,
-                                                       double *lo64, double *hi64, float *flo, float *fhi,
-                                                       float *bounds) {
+__device__ __forceinline__ void face_bounds(const MeshTopology &topo, const BroadphaseParams &p, const Axes &ax, int f,
+                                            double *lo, double *hi) {
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    lo[k] = INFINITY;
+    hi[k] = -INFINITY;
+  }
+  for (int j = 0; j < 3; j++) {
+    const int v = topo.faces[3 * f + j];
+    const int e0 = p.hoff ? p.hoff[v] : 0, e1 = p.hoff ? p.hoff[v + 1] : 2;
+    for (int e = e0; e < e1; e++) {
+      const double *src = entry_pos(p, v, e);
+      const double pos[3] = {src[0], src[1], src[2]};
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const double val = project<K>(pos, ax, k);
+        lo[k] = smin(val - p.eta, lo[k]);
+        hi[k] = smax(val + p.eta, hi[k]);
+      }
+    }
+  }
+}
+
+// A face with a marked vertex; out of line, off the other faces' registers.
+__device__ __noinline__ void marked_face_bounds(const MeshTopology &topo, const BroadphaseParams &p, const Axes &ax,
+                                                int f, double *lo, double *hi) {
+  face_bounds<13>(topo, p, ax, f, lo, hi);
+}
+
+template <int K>
+__global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, BroadphaseParams p, Axes ax,
+                                                       const double *vslab, double *lo64, double *hi64, float *flo,
+                                                       float *fhi, float *bounds) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   float cmin[3] = {INFINITY, INFINITY, INFINITY}, cmax[3] = {-INFINITY, -INFINITY, -INFINITY};
   if (f < topo.nf) {
     double lo[K], hi[K];
+    if constexpr (K == 13) {
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      lo[k] = INFINITY;
-      hi[k] = -INFINITY;
-    }
-    for (int j = 0; j < 3; j++) {
-      const int v = topo.faces[3 * f + j];
-      if (K == 13) {
+      for (int k = 0; k < K; k++) {
+        lo[k] = INFINITY;
+        hi[k] = -INFINITY;
+      }
+      bool marked = false;
+      for (int j = 0; j < 3; j++) {
+        const int v = topo.faces[3 * f + j];
         const double2 *q = reinterpret_cast<const double2 *>(vslab + (int64_t)kVertexSlab * v);
         double t[kVertexSlab];
 #pragma unroll
@@ -119,23 +177,24 @@ __global__ void __launch_bounds__(kThreads) leaf_slabs(MeshTopology topo, Broadp
           t[2 * k] = d.x;
           t[2 * k + 1] = d.y;
         }
+        marked = marked || t[0] > t[13];
 #pragma unroll
         for (int k = 0; k < K; k++) {
           lo[k] = smin(t[k], lo[k]);
           hi[k] = smax(t[13 + k], hi[k]);
         }
-        continue;
       }
-      const int e0 = p.hoff ? p.hoff[v] : 0, e1 = p.hoff ? p.hoff[v + 1] : 2;
-      for (int e = e0; e < e1; e++) {
-        const double *pos = p.hoff ? p.hpos + 3 * (int64_t)e : (e ? p.qe : p.qs) + 3 * (int64_t)v;
+      if (marked) {
+        double l[K], h[K];
+        marked_face_bounds(topo, p, ax, f, l, h);
 #pragma unroll
         for (int k = 0; k < K; k++) {
-          const double val = pos[k < 3 ? k : 0];  // AABBBroadPhase.cpp:38-39
-          lo[k] = smin(val - p.eta, lo[k]);
-          hi[k] = smax(val + p.eta, hi[k]);
+          lo[k] = l[k];
+          hi[k] = h[k];
         }
       }
+    } else {
+      face_bounds<K>(topo, p, ax, f, lo, hi);
     }
 #pragma unroll
     for (int k = 0; k < K; k++) {
@@ -1299,9 +1358,9 @@ int broadphase_run(const MeshTopology &topo, const BroadphaseParams &p, Broadpha
   if (kdop)
     vertex_slabs<<<grid_of(topo.nv), kThreads, 0, s>>>(topo.nv, p, ax, b.vslab);
   if (kdop)
-    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, b.vslab, b.lo64, b.hi64, flo, fhi, b.bounds);
+    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.vslab, b.lo64, b.hi64, flo, fhi, b.bounds);
   else
-    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, nullptr, b.lo64, b.hi64, flo, fhi, b.bounds);
+    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, nullptr, b.lo64, b.hi64, flo, fhi, b.bounds);
   BP_CUDA(cudaGetLastError());
   const KeyBits kb = key_bits(topo);
   // Refit only: the kept tree's leaf order and links stay, its node slabs are
@@ -1428,9 +1487,9 @@ int broadphase_enqueue_refit(const MeshTopology &topo, const BroadphaseParams &p
   if (kdop)
     vertex_slabs<<<grid_of(topo.nv), kThreads, 0, s>>>(topo.nv, p, ax, b.vslab);
   if (kdop)
-    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, b.vslab, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
+    leaf_slabs<13><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, b.vslab, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
   else
-    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, nullptr, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
+    leaf_slabs<3><<<grid_of(nf), kThreads, 0, s>>>(topo, p, ax, nullptr, b.lo64, b.hi64, b.face_lo, b.face_hi, b.bounds);
   const KeyBits kb = key_bits(topo);
   if (kdop)
     gather_leaves<13><<<grid_of(nf), kThreads, 0, s>>>(nf, b.keys, kb.fmask, b.face_lo, b.face_hi, b.leaf_box);
