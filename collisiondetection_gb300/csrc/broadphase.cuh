@@ -41,12 +41,17 @@ struct MeshTopology {
   // different instances are never paired.
   const int32_t *face_inst;    // [nf] instance of each face
   int32_t ninst;
+  // The vertices that faces use, nslab of them (slab_verts null: all, in
+  // order), and each face's corners as indices into that list.
+  int32_t nslab;
+  const int32_t *slab_verts;   // [nslab]
+  const int32_t *face_slabs;   // [nf][3]
 };
 
 // Device buffers of one broad-phase call; grown by the caller.
 struct BroadphaseBuffers {
   int64_t cap_faces = 0, cap_verts = 0, cap_pairs = 0;
-  double *vslab = nullptr;                        // [nv][26]   slabs of the vertices (13-DOP)
+  double *vslab = nullptr;                        // [cap_verts][26] slabs of the faces' vertices (13-DOP)
   // per face / node
   double *lo64 = nullptr, *hi64 = nullptr;        // [13][nf]
   float *face_lo = nullptr, *face_hi = nullptr;   // [13][nf]   outward-rounded FP32 slabs by face

@@ -87,6 +87,8 @@ struct ccd_mesh {
   int32_t *faces = nullptr, *face_rank = nullptr, *rank_triple = nullptr, *face_edges = nullptr,
           *rank_edge = nullptr;
   int32_t *face_inst = nullptr;  // instance of each face (meshes made of independent instances)
+  // the vertices that faces use and the faces' corners in that list (null: every vertex is used)
+  int32_t nslab = 0, *slab_verts = nullptr, *face_slabs = nullptr;
   int32_t ninst = 1;
   double *qs = nullptr, *qe = nullptr;
   // A multi-entry History (ccd_mesh_set_history), used instead of qs / qe
@@ -284,7 +286,8 @@ int narrow_device(ccd_mesh *m, Lane &L, int kind, int path, int64_t n, const int
 ccd::MeshTopology mesh_topology(const ccd_mesh *m, bool whole) {
   return ccd::MeshTopology{m->nv,        m->nf,        m->nranks,      m->nedges,
                            m->faces,     m->face_rank, m->rank_triple, m->face_edges,
-                           m->rank_edge, whole ? nullptr : m->face_inst, whole ? 1 : m->ninst};
+                           m->rank_edge, whole ? nullptr : m->face_inst, whole ? 1 : m->ninst,
+                           m->nslab,     m->slab_verts, m->slab_verts ? m->face_slabs : m->faces};
 }
 
 ccd::BroadphaseParams mesh_params(const ccd_mesh *m, int kind, double outer_eta) {
@@ -361,7 +364,7 @@ int check_eta(ccd_mesh *m, int64_t n, const double *eta, int64_t eta_count) {
 }
 
 void free_mesh_buffers(ccd_mesh *m) {
-  void *ptrs[] = {m->faces, m->face_rank, m->rank_triple, m->face_edges, m->rank_edge, m->face_inst, m->qs, m->qe,
+  void *ptrs[] = {m->faces, m->face_rank, m->rank_triple, m->face_edges, m->rank_edge, m->face_inst, m->slab_verts, m->face_slabs, m->qs, m->qe,
                   m->hist_off, m->hist_time, m->hist_pos, m->step_off, m->step_time, m->step_pos, m->fixed,
                   m->cand[0], m->cand[1], m->in_st, m->in_eta, m->which, m->d_eta,
                   m->col[0], m->col[1], m->col_t[0], m->col_t[1]};
@@ -423,6 +426,9 @@ int create_mesh(ccd_context *ctx, int32_t nverts, int32_t nfaces, const int32_t 
   if (!rc) rc = upload(&m->rank_triple, topo.rank_triple.data(), topo.rank_triple.size());
   if (!rc) rc = upload(&m->face_edges, topo.face_edges.data(), topo.face_edges.size());
   if (!rc) rc = upload(&m->rank_edge, topo.rank_edge.data(), topo.rank_edge.size());
+  m->nslab = topo.slab_verts.empty() ? nverts : (int32_t)topo.slab_verts.size();
+  if (!rc && !topo.slab_verts.empty()) rc = upload(&m->slab_verts, topo.slab_verts.data(), topo.slab_verts.size());
+  if (!rc && !topo.slab_verts.empty()) rc = upload(&m->face_slabs, topo.face_slabs.data(), topo.face_slabs.size());
   if (!rc && face_inst && ninst > 1) {
     rc = upload(&m->face_inst, face_inst->data(), face_inst->size());
     m->ninst = ninst;

@@ -11,6 +11,21 @@ namespace ccd {
 bool build_topology(int32_t nverts, int32_t nfaces, const int32_t *faces, HostTopology &out) {
   for (int64_t i = 0; i < 3 * (int64_t)nfaces; i++)
     if (faces[i] < 0 || faces[i] >= nverts) return false;
+  std::vector<int32_t> slab_of(nverts, -1);
+  for (int64_t i = 0; i < 3 * (int64_t)nfaces; i++) slab_of[faces[i]] = 0;
+  out.slab_verts.clear();
+  out.face_slabs.clear();
+  for (int32_t v = 0; v < nverts; v++)
+    if (slab_of[v] == 0) {
+      slab_of[v] = (int32_t)out.slab_verts.size();
+      out.slab_verts.push_back(v);
+    }
+  if ((int32_t)out.slab_verts.size() == nverts) {
+    out.slab_verts.clear();
+  } else {
+    out.face_slabs.resize(3 * (size_t)nfaces);
+    for (int64_t i = 0; i < 3 * (int64_t)nfaces; i++) out.face_slabs[i] = slab_of[faces[i]];
+  }
   struct Tri {
     int32_t a, b, c;
   };

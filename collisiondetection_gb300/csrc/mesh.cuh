@@ -12,9 +12,11 @@ namespace ccd {
 // Ranks of a mesh's faces and edges in lexicographic order (computed once per
 // mesh).  face_rank: rank of each face's ascending vertex triple (equal
 // triples share a rank); face_edges: rank of edge (v_i, v_{i+1 mod 3}) among
-// the ascending undirected edges.  Returns false on an out-of-range index.
+// the ascending undirected edges.  slab_verts: the vertices that faces use,
+// ascending, and face_slabs: the faces' corners as indices into it (both empty
+// when faces use every vertex).  Returns false on an out-of-range index.
 struct HostTopology {
-  std::vector<int32_t> face_rank, rank_triple, face_edges, rank_edge;
+  std::vector<int32_t> face_rank, rank_triple, face_edges, rank_edge, slab_verts, face_slabs;
 };
 bool build_topology(int32_t nverts, int32_t nfaces, const int32_t *faces, HostTopology &out);
 

@@ -1,7 +1,9 @@
 """The 13-DOP leaf slabs, formed from slabs per vertex, against the oracle's
-candidates where the two ways of forming them could part: NaN positions."""
+candidates where the two ways of forming them could part: NaN positions,
+vertices that few faces or none use."""
 import os
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -41,3 +43,54 @@ def test_nan_start_positions(orc, kind, share):
     ovf, oee = orc.broadphase(kind, q0, q1, f, 1e-6)
     for a, b in ((vf, ovf), (ee, oee), (again[0], ovf), (again[1], oee)):
         np.testing.assert_array_equal(a, b)
+
+
+def _soup(rng, n):
+    """n triangles that share no vertex."""
+    q0 = rng.random((n, 1, 3)) + 0.1 * rng.normal(size=(n, 3, 3))
+    q1 = q0 + 0.05 * rng.normal(size=(n, 1, 3))
+    return q0.ravel(), q1.ravel(), np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+
+
+@pytest.mark.parametrize("kind", [C.BROADPHASE_KDOP13, C.BROADPHASE_AABB])
+@pytest.mark.parametrize("mesh", ["bare", "bare_first", "soup", "pair"])
+def test_vertices_that_few_or_no_faces_use(orc, kind, mesh):
+    rng = np.random.default_rng(8)
+    if mesh == "soup":  # more than two vertices a face
+        q0, q1, f = _soup(rng, 600)
+    elif mesh == "pair":  # the smallest mesh with a tree
+        q0, q1, f = _soup(rng, 2)
+        q1 = q0.copy()
+        q1[9:] = q0[:9]
+    else:  # vertices that no face uses, after and between the others
+        q0, q1, f = W.two_spheres(3, level=2)
+        n = q0.size // 3
+        at = np.arange(n) if mesh == "bare" else np.sort(rng.permutation(3 * n)[:n])
+        a, b = rng.random((3 * n, 3)), rng.random((3 * n, 3))
+        a[at], b[at] = q0.reshape(-1, 3), q1.reshape(-1, 3)
+        q0, q1, f = a.ravel(), b.ravel(), at[f].astype(np.int32)
+    ovf, oee = orc.broadphase(kind, q0, q1, f, 1e-6)
+    with C.Context(0) as ctx, C.Mesh(ctx, f, q0, q1) as m:
+        for _ in range(2):  # a new tree, then the kept one
+            vf, ee = m.broadphase(kind, 1e-6)
+            np.testing.assert_array_equal(vf, ovf)
+            np.testing.assert_array_equal(ee, oee)
+
+
+def test_bare_vertices_cost_nothing():
+    # Two million vertices that no face uses beside 20,480 faces' own (1.6
+    # times the broad phase when every vertex had slabs).
+    q0, q1, f = W.two_spheres(1, level=5)
+    extra = np.random.default_rng(0).random(6_000_000) * 0.5
+
+    def median(a, b):
+        with C.Context(0) as ctx, C.Mesh(ctx, f, a, b) as m:
+            times = []
+            for _ in range(20):
+                t0 = time.perf_counter()
+                m.broadphase(C.BROADPHASE_KDOP13, 1e-6)
+                times.append(time.perf_counter() - t0)
+        return float(np.median(times[5:]))
+
+    q0, q1 = q0.ravel(), q1.ravel()
+    assert median(np.concatenate([q0, extra]), np.concatenate([q1, extra])) < 1.25 * median(q0, q1)
