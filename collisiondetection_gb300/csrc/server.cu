@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/ccd_gb300.h"
+#include "footprint.h"
 
 namespace {
 
@@ -32,14 +33,6 @@ using Clock = std::chrono::steady_clock;
 
 double ms_between(Clock::time_point a, Clock::time_point b) {
   return std::chrono::duration<double, std::milli>(b - a).count();
-}
-
-// Estimated device bytes of one request: topology and positions, broad-phase
-// buffers (slabs, tree, Morton keys, about 8 candidate face pairs per face and
-// their stencil keys) and the narrow-phase rows and refinement scratch of its
-// candidate stencils.
-int64_t footprint(const ccd_request &r) {
-  return (int64_t)4096 * r.nfaces + (int64_t)64 * r.nverts + ((int64_t)64 << 20);
 }
 
 struct Job {
@@ -208,7 +201,7 @@ int ccd_server_submit(ccd_server *s, const ccd_request *req, uint64_t *ticket) {
     if (job->faces[(size_t)i] < 0 || job->faces[(size_t)i] >= req->nverts) return CCD_ERR_INVALID_ARGUMENT;
   if (req->fixed) job->fixed.assign(req->fixed, req->fixed + req->nverts);
   job->frames = req->frames;
-  job->bytes = footprint(*req);
+  job->bytes = ccd::request_footprint(req->nfaces, req->nverts);
   job->submitted = Clock::now();
   {
     std::lock_guard<std::mutex> lock(s->mu);
