@@ -824,6 +824,7 @@ std::vector<uintptr_t> graph_signature(const ccd_mesh *m) {
       (uintptr_t)m->qs, (uintptr_t)m->qe, (uintptr_t)m->fixed, (uintptr_t)m->has_fixed, (uintptr_t)m->d_eta,
       (uintptr_t)m->cand[0], (uintptr_t)m->cand[1], (uintptr_t)m->col[0], (uintptr_t)m->col[1],
       (uintptr_t)m->col_t[0], (uintptr_t)m->col_t[1], (uintptr_t)m->side,
+      (uintptr_t)b.vslab, (uintptr_t)b.cap_verts,
       (uintptr_t)b.lo64, (uintptr_t)b.hi64, (uintptr_t)b.face_lo, (uintptr_t)b.face_hi, (uintptr_t)b.leaf_box,
       (uintptr_t)b.node_box, (uintptr_t)b.node_child, (uintptr_t)b.node_links, (uintptr_t)b.leaf_links,
       (uintptr_t)b.leaf_end, (uintptr_t)b.parent, (uintptr_t)b.arrive, (uintptr_t)b.keys, (uintptr_t)b.counters,
