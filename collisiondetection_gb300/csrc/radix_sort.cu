@@ -155,9 +155,8 @@ constexpr int64_t kGridPer = 2048;                  // keys per block at least
 constexpr int64_t kGridMaxKeys = (int64_t)1 << 22;
 constexpr int kGridMaxBlocks = 256;
 
-__global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals,
-                                                          uint32_t *vals_alt, int64_t n, int begin_bit, int end_bit,
-                                                          uint32_t *counts) {
+__global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64_t *keys_alt, int64_t n, int begin_bit,
+                                                          int end_bit, uint32_t *counts) {
   namespace cg = cooperative_groups;
   cg::grid_group grid = cg::this_grid();
   __shared__ uint32_t warp_hist[kGridWarps][256];
@@ -168,28 +167,24 @@ __global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64
   const int64_t run0 = ((int64_t)blockIdx.x * kGridWarps + warp) * run;
   const int64_t run1 = run0 + run < n ? run0 + run : n;
   uint64_t *src = keys, *dst = keys_alt;
-  uint32_t *vsrc = vals, *vdst = vals_alt;
   int pass = 0;
   for (int shift = begin_bit; shift < end_bit; shift += 8, pass++) {
     for (int i = tid; i < kGridWarps * 256; i += kGridThreads) (&warp_hist[0][0])[i] = 0;
     __syncthreads();
     for (int64_t k = run0 + lane; k < run1; k += 32) atomicAdd(&warp_hist[warp][(src[k] >> shift) & 255u], 1u);
     __syncthreads();
-    // Two sets of counts: the next pass writes its own while a block still
-    // reads this one's.
-    uint32_t *mine = counts + (size_t)(pass & 1) * kGridMaxBlocks * 256;
     if (tid < 256) {
       uint32_t c = 0;
 #pragma unroll
       for (int w = 0; w < kGridWarps; w++) c += warp_hist[w][tid];
-      mine[(size_t)blockIdx.x * 256 + tid] = c;
+      counts[(size_t)blockIdx.x * 256 + tid] = c;
     }
     grid.sync();
     uint32_t before = 0, total = 0, x = 0;
     if (tid < 256) {
 #pragma unroll 8
       for (int b = 0; b < nblocks; b++) {
-        const uint32_t c = __ldcg(mine + (size_t)b * 256 + tid);
+        const uint32_t c = __ldcg(counts + (size_t)b * 256 + tid);
         total += c;
         if (b < (int)blockIdx.x) before += c;
       }
@@ -225,24 +220,16 @@ __global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64
       __syncwarp();
       if (valid && (peers & lt) == 0) warp_hist[warp][d] += __popc(peers);
       __syncwarp();
-      if (valid) {
-        dst[pos] = key;
-        if (vals) vdst[pos] = vsrc[k];
-      }
+      if (valid) dst[pos] = key;
     }
     grid.sync();
     uint64_t *t = src;
     src = dst;
     dst = t;
-    uint32_t *tv = vsrc;
-    vsrc = vdst;
-    vdst = tv;
   }
   if (pass & 1) {
-    for (int64_t k = (int64_t)blockIdx.x * kGridThreads + tid; k < n; k += (int64_t)nblocks * kGridThreads) {
+    for (int64_t k = (int64_t)blockIdx.x * kGridThreads + tid; k < n; k += (int64_t)nblocks * kGridThreads)
       keys[k] = src[k];
-      if (vals) vals[k] = vsrc[k];
-    }
   }
 }
 
@@ -292,7 +279,7 @@ cudaError_t exclusive_scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uin
 
 size_t radix_sort_temp_bytes(int64_t n) {
   const int64_t nblocks = (n + kTile - 1) / kTile;
-  const int64_t m = std::max<int64_t>(256 * nblocks, 256 * kGridMaxBlocks);  // sort_grid: two sets of counts
+  const int64_t m = std::max<int64_t>(256 * nblocks, 256 * kGridMaxBlocks);  // sort_grid: 256 counts per block
   return 2 * align_up((size_t)m * sizeof(uint32_t)) + scan_temp_bytes(m);
 }
 
@@ -302,7 +289,7 @@ cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, u
   if (n >= (int64_t)1 << 31 || temp_bytes < radix_sort_temp_bytes(n)) return cudaErrorInvalidValue;
   const int64_t nblocks = (n + kTile - 1) / kTile;
   const int64_t m = 256 * nblocks;
-  if (n <= kGridMaxKeys) {
+  if (!vals && n <= kGridMaxKeys) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -310,7 +297,7 @@ cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, u
     const int most = std::min(sms, kGridMaxBlocks);
     const int grid = (int)std::min<int64_t>((n + kGridPer - 1) / kGridPer, most);
     uint32_t *counts = (uint32_t *)temp;
-    void *args[] = {&keys, &keys_alt, &vals, &vals_alt, &n, &begin_bit, &end_bit, &counts};
+    void *args[] = {&keys, &keys_alt, &n, &begin_bit, &end_bit, &counts};
     return cudaLaunchCooperativeKernel((const void *)sort_grid, dim3(grid), dim3(kGridThreads), args, 0, s);
   }
   uint32_t *counts = (uint32_t *)temp;
