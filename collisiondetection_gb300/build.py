@@ -21,7 +21,7 @@ CU_SOURCES = ["narrow_vf.cu", "narrow_ee.cu", "narrow_vevv.cu", "narrow.cu", "qu
               "broadphase.cu", "mesh.cu", "capi.cu", "capi_mesh.cu",
               "capi_noalloc.cu", "capi_tune.cu", "server.cu", "distance.cu", "penalty.cu", "separating.cu", "velocity.cu"]
 HEADERS = ["ccd_common.h", "ccd_math.h", "ccd_math_tables.h", "ccd_jt.h", "ccd_jt_warp.h", "ccd_jt_shifts.h", "ccd_ctcd64.h", "ccd_classify.h", "ccd_div.h", "ccd_cull32.h", "narrow.cuh", "narrow_kernels.cuh", "stages.cuh",
-           "radix_sort.cuh", "broadphase.cuh", "mesh.cuh", "context.cuh", "ccd_distance.h", "distance.cuh", "separating.cuh", "penalty.cuh", "velocity.cuh", "ccd_heap.h",
+           "radix_sort.cuh", "sort_rule.h", "broadphase.cuh", "mesh.cuh", "context.cuh", "ccd_distance.h", "distance.cuh", "separating.cuh", "penalty.cuh", "velocity.cuh", "ccd_heap.h",
            "footprint.h"]
 
 NVCC_FLAGS = [

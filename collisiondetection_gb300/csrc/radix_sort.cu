@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "radix_sort.cuh"
+#include "sort_rule.h"
 
 namespace ccd {
 
@@ -149,11 +150,7 @@ __global__ void __launch_bounds__(kThreads) digit_scatter(const uint64_t *keys, 
 // of 38 bits: 2^12 keys 111 and 40 us, 2^16 136 and 45, 2^20 210 and 108, 2^22
 // 339 and 258, 2^23 693 and 768 (one block per SM no longer keeps enough of its
 // range in flight), so the line lies at 2^22.
-constexpr int kGridThreads = 512;
 constexpr int kGridWarps = kGridThreads / 32;
-constexpr int64_t kGridPer = 2048;                  // keys per block at least
-constexpr int64_t kGridMaxKeys = (int64_t)1 << 22;
-constexpr int kGridMaxBlocks = 256;
 
 __global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64_t *keys_alt, int64_t n, int begin_bit,
                                                           int end_bit, uint32_t *counts) {
@@ -290,15 +287,22 @@ cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, u
   const int64_t nblocks = (n + kTile - 1) / kTile;
   const int64_t m = 256 * nblocks;
   if (!vals && n <= kGridMaxKeys) {
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, cooperative = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sort_grid, kGridThreads, 0);
     if (e != cudaSuccess) return e;
-    const int most = std::min(sms, kGridMaxBlocks);
-    const int grid = (int)std::min<int64_t>((n + kGridPer - 1) / kGridPer, most);
-    uint32_t *counts = (uint32_t *)temp;
-    void *args[] = {&keys, &keys_alt, &n, &begin_bit, &end_bit, &counts};
-    return cudaLaunchCooperativeKernel((const void *)sort_grid, dim3(grid), dim3(kGridThreads), args, 0, s);
+    const int grid = grid_sort_blocks(n, cooperative != 0, sms, per_sm);
+    if (grid > 0) {
+      uint32_t *counts = (uint32_t *)temp;
+      void *args[] = {&keys, &keys_alt, &n, &begin_bit, &end_bit, &counts};
+      e = cudaLaunchCooperativeKernel((const void *)sort_grid, dim3(grid), dim3(kGridThreads), args, 0, s);
+      // a context that may use part of the SMs only refuses what it cannot
+      // hold at once: the passes then follow one by one
+      if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+      cudaGetLastError();
+    }
   }
   uint32_t *counts = (uint32_t *)temp;
   uint32_t *offsets = (uint32_t *)((char *)temp + align_up((size_t)m * sizeof(uint32_t)));
