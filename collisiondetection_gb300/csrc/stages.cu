@@ -44,13 +44,13 @@ StageScratch stage_scratch_view(void *base, int64_t cap) {
   sc.wave_steps = 0;
   sc.wave_min_rows = 0;
   sc.pool_budget = 0;
-  sc.warp_finish = 1;
+  sc.warp_finish = kWarpFinish;
   sc.shift_after = kShiftAfter;
   sc.finish_shift_after = kFinishShiftAfter;
-  sc.pool_slots = stages::kWarpPool;
-  sc.pool_slots_min = stages::kWarpPool;
+  sc.pool_slots = kPoolSlots;
+  sc.pool_slots_min = kPoolSlotsMin;
   sc.pool_all = 0;
-  sc.pool_phase_sync = 0;
+  sc.pool_phase_sync = kPoolPhaseSync;
   return sc;
 }
 

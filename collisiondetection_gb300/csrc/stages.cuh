@@ -79,6 +79,10 @@ inline void resolve_split(bool vf, int64_t rows, int &steps, int &budget) {
 // Failed shifts before a stage's remaining ones run at once: in the pool, and
 // in the one-per-warp finish, whose solves have failed some already.
 constexpr int kShiftAfter = 2, kFinishShiftAfter = 1;
+// The other defaults of a context and of the allocation-free call: the slowest
+// solves on whole warps with a stage's shifts at once; 64 slots a warp, of which
+// a small batch fills one; warps on the phase of the SM clock's 2^16 cycles.
+constexpr int kWarpFinish = 2, kPoolSlots = 64, kPoolSlotsMin = 1, kPoolPhaseSync = 16;
 // Job lists: one per (working phase, current degree 3..6).
 constexpr int kWaveBins = 16;
 
