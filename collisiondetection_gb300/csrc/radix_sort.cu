@@ -2,6 +2,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "radix_sort.cuh"
 #include "sort_rule.h"
@@ -230,6 +231,28 @@ __global__ void __launch_bounds__(kGridThreads) sort_grid(uint64_t *keys, uint64
   }
 }
 
+// Blocks of sort_grid that the current device runs at once, at most one per SM;
+// asked once per device (the occupancy query takes longer than a launch).
+cudaError_t resident_blocks(int *most) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];  // blocks + 1; 0: not asked yet
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < kDevices && known[dev].load() > 0) {
+    *most = known[dev].load() - 1;
+    return cudaSuccess;
+  }
+  int sms = 0, cooperative = 0, per_sm = 0;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sort_grid, kGridThreads, 0);
+  if (e != cudaSuccess) return e;
+  *most = grid_sort_limit(cooperative != 0, sms, per_sm);
+  if (dev >= 0 && dev < kDevices) known[dev].store(*most + 1);
+  return cudaSuccess;
+}
+
 }  // namespace
 
 size_t scan_temp_bytes(int64_t n) {
@@ -287,13 +310,10 @@ cudaError_t radix_sort_u64(uint64_t *keys, uint64_t *keys_alt, uint32_t *vals, u
   const int64_t nblocks = (n + kTile - 1) / kTile;
   const int64_t m = 256 * nblocks;
   if (!vals && n <= kGridMaxKeys) {
-    int dev = 0, sms = 0, cooperative = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sort_grid, kGridThreads, 0);
+    int most = 0;
+    cudaError_t e = resident_blocks(&most);
     if (e != cudaSuccess) return e;
-    const int grid = grid_sort_blocks(n, cooperative != 0, sms, per_sm);
+    const int grid = grid_sort_blocks(n, most);
     if (grid > 0) {
       uint32_t *counts = (uint32_t *)temp;
       void *args[] = {&keys, &keys_alt, &n, &begin_bit, &end_bit, &counts};
