@@ -188,12 +188,8 @@ namespace stages {
 // of 3.38, a cloth step of 211,970 faces 1.50 instead of 1.40.
 __device__ __forceinline__ void follow() { cudaGridDependencySynchronize(); }
 
-// All of these kernels ask for the pool's division of an SM between L1 and
-// shared memory: an SM changes it only when idle, which it never is between
-// kernels launched this way, and the pool's blocks that do not fit wait for the
-// first ones to end.  (A cloth step in contact, two streams: 2.14 -> 1.70 ms.)
 template <class... P, class... A>
-void launch_next(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+void launch_after(void (*kernel)(P...), int grid, int threads, size_t smem, bool pool_split, cudaStream_t s, A... args) {
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attrs[0].val.programmaticStreamSerializationAllowed = 1;
@@ -205,8 +201,25 @@ void launch_next(void (*kernel)(P...), int grid, int threads, size_t smem, cudaS
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attrs;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pool_split ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // run() returns the last error
+}
+
+// The pool and the kernels around it all ask for the pool's division of an SM
+// between L1 and shared memory: an SM changes it only when idle, which it never
+// is between kernels launched this way, and the pool's blocks that do not fit
+// wait for the first ones to end.  (A cloth step in contact, two streams: 2.14
+// -> 1.70 ms.)
+template <class... P, class... A>
+void launch_next(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  launch_after(kernel, grid, threads, smem, true, s, args...);
+}
+
+// The wavefront's kernels keep the L1 for the solver states they gather, and its
+// finish for the states in its lanes' local memory.
+template <class... P, class... A>
+void launch_wave(void (*kernel)(P...), int grid, int threads, cudaStream_t s, A... args) {
+  launch_after(kernel, grid, threads, 0, false, s, args...);
 }
 
 __device__ __forceinline__ void store_spans(const StageScratch &sc, int slot, int64_t r, const SpanList &sl) {
@@ -1008,14 +1021,14 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
       // counts: 3 rotating sets, then the tail and spill lengths
       e = cudaMemsetAsync(sc.wcount, 0, (3 * kWaveBins + 2) * sizeof(unsigned), s);
       if (e != cudaSuccess) return e;
-      launch_next(wave_start<Polys>, wave_grid, kWaveThreads, 0, s, sc);
+      launch_wave(wave_start<Polys>, wave_grid, kWaveThreads, s, sc);
       for (int it = 0; it < steps; it++) {
-        launch_next(wave_step<Polys>, wave_grid, kWaveThreads, 0, s, sc, sc.wlist + (it & 1) * lstride,
+        launch_wave(wave_step<Polys>, wave_grid, kWaveThreads, s, sc, sc.wlist + (it & 1) * lstride,
                     sc.wcount + kWaveBins * (it % 3), sc.wlist + ((it + 1) & 1) * lstride,
                     sc.wcount + kWaveBins * ((it + 1) % 3), sc.wcount + kWaveBins * ((it + 2) % 3));
       }
       unsigned *tcount = sc.wcount + 3 * kWaveBins, *scount = tcount + 1;
-      launch_next(wave_gather_tail<Polys>, num_sms, kWaveThreads, 0, s, sc, sc.wlist + (steps & 1) * lstride,
+      launch_wave(wave_gather_tail<Polys>, num_sms, kWaveThreads, s, sc, sc.wlist + (steps & 1) * lstride,
                   sc.wcount + kWaveBins * (steps % 3), tcount);
       // The unfinished jobs continue in the pool kernel (many per warp); the
       // few that exceed its step budget finish one per warp, as many warps as
@@ -1025,7 +1038,7 @@ cudaError_t run(const PrimBatch &b, const int32_t *list, const StageScratch &sc,
                   PoolJobs{sc.tail, tcount, budget, sc.wlist, scount});
       StageScratch last = sc;
       last.shift_after = sc.finish_shift_after;
-      launch_next(wave_finish<Polys>, num_sms * 32, 32, 0, s, last, sc.wlist, scount);
+      launch_wave(wave_finish<Polys>, num_sms * 32, 32, s, last, sc.wlist, scount);
       *launches += steps + 4;
     } else {
       if (sc.pool_slots == 32)
