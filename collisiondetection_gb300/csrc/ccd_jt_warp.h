@@ -592,11 +592,41 @@ struct Solve {
     type = s.I(TYPE), flags = s.I(FLAGS), jq = s.I(JQ), jr = s.I(JR), roots = s.I(ROOTS), status = s.I(STATUS);
   }
 
-  // Runs the solve to its end; every lane receives the roots in tr[0 .. 5].
-  __device__ __forceinline__ void run(double (&tr)[6]) {
-    while (mode != kDone) step();
+  // The state to storage of ccd_jt.h, whole in every lane's own.
+  __device__ __forceinline__ void store(LocalStorage &st) const {
+    const LocalState s{&st};
+    for (int i = 0; i < 7; i++) {
+      s.D(P + i) = at(p, i);
+      s.D(QP + i) = at(qp, i);
+    }
+    for (int i = 0; i < 6; i++) {
+      s.D(K + i) = at(k, i);
+      s.D(QK + i) = at(qk, i);
+      s.D(SVK + i) = at(svk, i);
+      s.D(TEMP + i) = at(temp, i);
+      s.Z(i) = at(zr, i);
+    }
+    s.D(U) = u, s.D(V) = v, s.D(A) = a, s.D(B) = b, s.D(C) = c, s.D(DD) = d;
+    s.D(A1) = a1, s.D(A3) = a3, s.D(A7) = a7, s.D(E) = e, s.D(F) = f, s.D(G) = g, s.D(H) = h;
+    s.D(BND) = bnd, s.D(XX) = xx, s.D(YY) = yy;
+    s.D(SVU) = svu, s.D(SVV) = svv, s.D(XS) = xs, s.D(BETAS) = betas, s.D(BETAV) = betav;
+    s.D(OSS) = oss, s.D(OVV) = ovv, s.D(OTS) = ots, s.D(OTV) = otv;
+    s.D(VV) = vv, s.D(SS) = ss, s.D(TV) = tv, s.D(TS) = ts, s.D(UI) = ui, s.D(VI) = vi;
+    s.D(RELSTP) = relstp, s.D(OMP) = omp, s.D(RX) = rx, s.D(RT) = rt;
+    s.I(MODE) = mode, s.I(N) = n, s.I(DEG) = deg, s.I(CNT) = cnt, s.I(J) = j, s.I(L2) = l2;
+    s.I(TYPE) = type, s.I(FLAGS) = flags, s.I(JQ) = jq, s.I(JR) = jr, s.I(ROOTS) = roots, s.I(STATUS) = status;
+  }
+
+  // Runs the solve until it is done (true; every lane receives the roots in
+  // tr[0 .. 5]) or in shift number `after` of a stage (false).
+  __device__ __forceinline__ bool run(double (&tr)[6], int after) {
+    while (mode != kDone) {
+      if (mode != kInit && cnt >= after) return false;
+      step();
+    }
 #pragma unroll
     for (int i = 0; i < 6; i++) tr[i] = at(zr, i);
+    return true;
   }
 };
 

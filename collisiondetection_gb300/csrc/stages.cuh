@@ -77,8 +77,12 @@ inline void resolve_split(bool vf, int64_t rows, int &steps, int &budget) {
   if (budget == kBySize) budget = brief ? 0 : kPoolBudget;
 }
 // Failed shifts before a stage's remaining ones run at once: in the pool, and
-// in the one-per-warp finish, whose solves have failed some already.
-constexpr int kShiftAfter = 2, kFinishShiftAfter = 1;
+// in the one-per-warp finish, whose solves have failed some already.  In the
+// pool a stage that its fifth shift or an earlier one ends is faster one by one
+// (65,537 edge-edge rows, slow seeds: 19.1, 17.7, 15.2 ms with 2, 11.8, 12.3,
+// 11.4 with 5), and one that fails them all loses little (1,000 flat rows 16.8
+// and 21.0 ms, with 12 42.6).
+constexpr int kShiftAfter = 5, kFinishShiftAfter = 1;
 // The other defaults of a context and of the allocation-free call: the slowest
 // solves on whole warps with a stage's shifts at once; 64 slots a warp, of which
 // a small batch fills one; warps on the phase of the SM clock's 2^16 cycles.
@@ -441,32 +445,30 @@ __device__ __forceinline__ void finish_job(const StageScratch &sc, const S &st, 
   finish_roots<Polys>(sc, slot, j, tr, st.I(jt::ROOTS), st.I(jt::STATUS));
 }
 
-// The solve of state st run to its end by the whole (converged) warp
-// (ccd_jt_warp.h); lane 0 writes its spans.
-template <class Polys, class S>
-__device__ __forceinline__ void warp_solve(const StageScratch &sc, const S &st, int slot, int64_t j) {
-  jt::warp::Solve ws;
-  ws.load(st);
-  double tr[6];
-  ws.run(tr);
-  if ((threadIdx.x & 31) == 0) finish_roots<Polys>(sc, slot, j, tr, ws.roots, ws.status);
-}
-
 __device__ __forceinline__ int job_queue(const int *qbase, int nslots, int64_t g) {
   int q = 0;
   while (q + 1 < nslots && g >= qbase[q + 1]) q++;
   return q;
 }
 
-// The solve of state st run to its end by the whole warp, each lane trying
-// one of the stage's remaining shifts (ccd_jt_shifts.h); lane 0 writes its
-// spans.
+// The solve of state st run to its end by the whole (converged) warp: with its
+// independent operations on different lanes (ccd_jt_warp.h), and, warp_finish
+// 2, from the shift_after-th shift of a stage on with each lane trying one of
+// the stage's remaining shifts (ccd_jt_shifts.h).  Lane 0 writes its spans.
+// (The second way from the start, one lane's operations on all of them, takes
+// longer on solves that fail few shifts or none: 4,096 vertex-face rows, mean
+// of 60 batches, 753 us and now 685.)
 template <class Polys, class S>
-__device__ __forceinline__ void shift_solve(const StageScratch &sc, const S &st, int slot, int64_t j) {
+__device__ __forceinline__ void solve_alone(const StageScratch &sc, const S &st, int slot, int64_t j) {
+  jt::warp::Solve ws;
+  ws.load(st);
+  double tr[6];
+  if (ws.run(tr, sc.warp_finish == 2 ? sc.shift_after : jt::shifts::kShifts)) {
+    if ((threadIdx.x & 31) == 0) finish_roots<Polys>(sc, slot, j, tr, ws.roots, ws.status);
+    return;
+  }
   jt::LocalStorage ls;
-  for (int f = 0; f < jt::kDoubles; f++) ls.d[f] = st.D(f);
-  for (int f = 0; f < jt::kInts; f++) ls.i[f] = st.I(f);
-  for (int k = 0; k < 6; k++) ls.zr[k] = st.Z(k);
+  ws.store(ls);
   jt::shifts::run(ls, sc.shift_after);
   if ((threadIdx.x & 31) == 0) finish_job<Polys>(sc, jt::LocalState{&ls}, slot, j);
 }
@@ -531,7 +533,6 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
   };
   int *mode = pool_i + jt::MODE * POOL;
   bool exhausted = njobs == 0;
-  int turns = 0;
   for (;;) {
     // Write out finished solves.
     for (int k = lane; k < POOL; k += 32) {
@@ -627,15 +628,7 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
         bestc = c;
       }
     }
-    bool alone = exhausted && working == 1 && sc.warp_finish;
-    // In a batch of a solve a warp, every solve is its warp's last from the
-    // start: there the warp takes over once the solve has failed the shifts
-    // that are tried one by one (looked at now and then).  Until then one lane
-    // on shared memory is the faster way: 4,096 vertex-face rows 0.50 and 0.47
-    // ms (0.48 with a look at every step).
-    if (alone && lim == 1 && sc.warp_finish == 2)
-      alone = (++turns & 63) == 0 && mode[0] != jt::kInit && pool_i[jt::CNT * POOL] >= sc.shift_after;
-    if (alone) {
+    if (exhausted && working == 1 && sc.warp_finish) {
       // The warp's last unfinished solve, with no job left to take: all 32
       // lanes copy its state and advance it together to the end
       // (jt::warp::step, or one shift per lane), then lane 0 writes it out.
@@ -647,10 +640,7 @@ __global__ void __launch_bounds__(32) stage_roots(StageScratch sc, PoolJobs pj) 
       }
       const int64_t g = job_of[k];
       const int q = job_queue(qbase, Polys::kSlots, g);
-      if (sc.warp_finish == 2)
-        shift_solve<Polys>(sc, state(k), q, g - qbase[q]);
-      else
-        warp_solve<Polys>(sc, state(k), q, g - qbase[q]);
+      solve_alone<Polys>(sc, state(k), q, g - qbase[q]);
       __syncwarp();
       if (lane == 0) mode[k] = jt::kEmpty;
       __syncwarp();
@@ -857,10 +847,8 @@ __global__ void __launch_bounds__(kWaveThreads) wave_gather_tail(StageScratch sc
 // The jobs the wavefront steps left unfinished, one per warp, each run to
 // its end (the solver's own iteration limits bound the loop).  Few jobs
 // remain by then and each is a long sequential chain, so latency, not lane
-// use, matters here.  With sc.warp_finish the warp holds the state in
-// registers spread over its lanes and advances the solve together
-// (jt::warp::Solve: element-wise updates and independent divisions on
-// different lanes); otherwise lane 0 runs it alone from a private copy.
+// use, matters here.  With sc.warp_finish the warp advances the solve together
+// (solve_alone); otherwise lane 0 runs it alone from a private copy.
 template <class Polys>
 __global__ void __launch_bounds__(32) wave_finish(StageScratch sc, const uint32_t *tail, const unsigned *tcount) {
   follow();
@@ -875,10 +863,8 @@ __global__ void __launch_bounds__(32) wave_finish(StageScratch sc, const uint32_
     int q;
     int64_t j;
     const jt::FieldState fs = wave_state<Polys>(sc, qbase, g, q, j);
-    if (sc.warp_finish == 2) {
-      shift_solve<Polys>(sc, fs, q, j);
-    } else if (whole) {
-      warp_solve<Polys>(sc, fs, q, j);
+    if (whole) {
+      solve_alone<Polys>(sc, fs, q, j);
     } else {
       jt::LocalStorage st;
       load_state(fs, st);

@@ -154,7 +154,7 @@ int ccd_last_batch_timings(ccd_context *ctx, ccd_batch_timings *out);
  *                    same results as the sequential order); default 2
  *   "shift_after"    warp_finish 2: shifts of a stage tried one at a time
  *                    before the remaining ones run at once; in [0, 19],
- *                    default 2, and 1 by the one-per-warp finish
+ *                    default 5, and 1 by the one-per-warp finish
  *   "chunk_rows"     ccd_prim_batch: largest chunk (rows) streamed through
  *                    the device, two in flight; a batch is cut into equal
  *                    chunks; in [1024, 2^26], default 2^23
