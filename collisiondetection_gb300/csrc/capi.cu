@@ -112,8 +112,8 @@ int collect_phase(ccd_context *ctx, PhaseEvents &pe) {
   return CCD_OK;
 }
 
-// The scratch with the context's solver options.  CCD_PATH_REFINE_ALL solves
-// every polynomial (classify false).
+// The scratch with the context's solver options.  classify false
+// (CCD_PATH_REFINE_ALL): every polynomial is solved.
 static ccd::StageScratch stage_view(const ccd_context *ctx, const StageBuf &stage, bool classify) {
   ccd::StageScratch view = stage.view;
   view.classify = classify;

@@ -22,9 +22,9 @@
 //     address and the SM count with that device current); make that first
 //     call before any stream capture that should contain later calls;
 //   * the only scratch that must start at zero is the batch counter block,
-//     which each call clears on the caller's stream before its kernels (the
-//     staged refinement clears its own job queues per tile; every other
-//     scratch array is written before it is read).
+//     which each call clears on the caller's stream before its kernels, with
+//     the first tile's job queues (the staged refinement clears those of the
+//     later tiles; every other scratch array is written before it is read).
 #include <cuda_runtime.h>
 #include <stdint.h>
 

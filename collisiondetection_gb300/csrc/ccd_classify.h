@@ -34,11 +34,13 @@
 // with a double root r beside a double root near -r: those came out up to 5e-3
 // off where the moduli agreed to 1%, and at most 1.5e-3 elsewhere, |p| < 1e-7.
 // A row is left to the solver when its sextic is below kMirror on the mirror
-// image of a cell on which it is below kMargin.  On the host
-// (tests/test_classify_host.py draws the same families), 130 M rows of eleven
-// families -- random, integer lattices, coplanar, parallel, tangential, flat
-// sheets, scales from 1e-6 to 1e4 -- gave no row that the full solve decides
-// otherwise, and no contact time that differs in a bit.
+// image of a cell on which it is below kMargin (from the fifth cell on: a
+// contact earlier than that has its mirror image among the start's cells).  On
+// the host (tests/test_classify_host.py and test_classify_edges_host.py draw
+// the same families), 137 M rows of twelve families -- random, integer
+// lattices, coplanar, parallel, tangential, flat sheets, scales from 1e-6 to
+// 1e4, mirrored roots from t = 5e-5 on -- gave no row that the full solve
+// decides otherwise, and no contact time that differs in a bit.
 #pragma once
 
 #include <string.h>
@@ -139,8 +141,8 @@ struct Row {
   }
 
   // Cells of one lane (bit i: cell 8 * lane + i) on which the sextic may be
-  // <= kMargin; mirrored: on the mirror image of one of them, a cell or more
-  // from the start, it may be <= kMirror.
+  // <= kMargin; mirrored: on the mirror image of one of them, four cells or
+  // more from the start, it may be <= kMirror.
   static CCD_HD unsigned near_contact(const float *w, int lane, bool &mirrored) {
     const float t0 = (float)(lane * kPer) * kCell;
     unsigned open = 0;
